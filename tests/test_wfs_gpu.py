@@ -180,3 +180,51 @@ def test_widest_subaperture_window_matches_oracle():
     ref = wfs_oracle.geom_grads(geom, layers, dms, 9, s.cfg.sim_dt, seed=3)
     assert rel(g, ref) < TOL
     W.close()
+
+
+@pytest.mark.parametrize("points, atm_dx, dense", [(6, 0.2, False), (6, 0.2, True), (26, 0.05, False),
+                                                   (26, 0.079, False), (26, 0.2, True), (34, 0.2, True),
+                                                   (34, 0.079, False)])
+def test_every_kind_of_stencil_matches_oracle(points, atm_dx, dense):
+    """Separable tiles, non-zero point lists and whole windows: the narrowest
+    and the widest windows, maps just within and beyond the pixels a separable
+    window spans (0.4 m windows on 0.079 m and 0.05 m pixels), and stencils
+    without zeros; DMs whose edge the windows cross; two instances."""
+    import dataclasses
+
+    import torch
+    from conftest import get_fit, get_system
+    from maos_b200 import wfs_setup
+    from maos_b200.turbulence import FrozenFlowAtmosphere
+    from maos_b200.wfs import GeomWfs
+    from oracle import wfs_oracle
+    s, fit = get_system("scao_8m"), get_fit("scao_8m")
+    geom = wfs_setup.build_geom_wfs(s, sim_dx=s.wfs[0].dsa / points)
+    P = geom.powfs[0]
+    assert P.nxsa == points
+    rng = np.random.default_rng(points)
+    if dense:
+        geom.powfs[0] = P = dataclasses.replace(P, stencils=P.stencils + rng.standard_normal(P.stencils.shape) * 1e-3)
+    cfg = dataclasses.replace(s.cfg, atm_dx=atm_dx)
+    atms = [FrozenFlowAtmosphere(cfg, 6 + i) for i in range(2)]
+    # a DM that ends inside the pupil: windows on, across and beyond its edge
+    n, dx = fit.dms[0].amap.nx - 6, fit.dms[0].amap.dx
+    a0 = atms[0]
+    layers = [(a0.n, a0.n, a0.dx, -a0.n / 2 * a0.dx, -a0.n / 2 * a0.dx, float(h), float(a0.vx[l]), float(a0.vy[l]))
+              for l, h in enumerate(cfg.atm_ht)]
+    W = GeomWfs(geom, layers, [(n, n, dx, -3.0, -2.9, 0.0)], cfg.sim_dt, nbatch=2)
+    for i, a in enumerate(atms):
+        W.set_atmosphere(i, a)
+    cmd = (rng.standard_normal((2, n * n)) * 1e-7).astype(np.float32)
+    g = W.grad(11, dm=torch.as_tensor(cmd, device="cuda")).cpu().numpy()
+    for i, a in enumerate(atms):
+        scr, _ = _screens(a)
+        # some points lie exactly on the DM's first row, where the last bit of the coordinate decides whether
+        # they count: the gradients that a shift of 1e-9 m either way changes are left out
+        c = cmd[i].reshape(n, n).astype(np.float64)
+        ref, up, down = (wfs_oracle.geom_grads(geom, scr, [wfs_oracle.Screen(c, -3.0, -2.9 + e, dx, 0.0)], 11,
+                                               cfg.sim_dt) for e in (0, 1e-9, -1e-9))
+        sure = np.abs(up - down) <= 1e-6 * np.abs(ref).max()
+        assert sure.mean() > 0.75
+        assert rel(g[i][sure], ref[sure]) < TOL
+    W.close()
