@@ -114,6 +114,7 @@ static void launch_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t
 // on the host, from which the padded gather lists of the kernels are built.
 struct RayTables {
     DevBuf<AxisW> fwd;
+    std::vector<AxisW> h_fwd;
     std::vector<int> h_ptr, h_idxptr;
     std::vector<GatherW> h_ent;
 };
@@ -127,22 +128,24 @@ struct Recon {
     int maxit = 0, precond = 0, split = 1;
     int nsc = 0;            // scalars per instance
     int nblk_x = 0;         // blocks over nxtot
-    int hxt_threads = kThreads, nblk_hxt = 0;  // k_hxt_rows's CTA size (autotuned) and CTAs per instance
     int nblk_tt = 0;        // blocks over the largest nsa
     std::vector<long> xoff, goff;
     std::vector<int> nsa;
 
     // tables
     RayTables hx;
-    // separable Hx^T: fixed-width transposed lists and the pupil-row buffer
-    DevBuf<GatherW> xpad, ypad;
-    DevBuf<int4> footprint;
-    int kx = 0, ky = 0, maxnx = 0, maxny = 0;
-    int prows = 0, ptiles = 0, ncols = 0;  // pupil rows per CTA, CTAs per WFS, sum of layer widths
-    long tw = 0;                           // row-buffer floats per (instance, WFS)
+    // k_pupil_rows: pupil rows per CTA, CTAs per WFS, the layer rows each touches
+    int prows = 0, ptiles = 0, pvrows = 0;
     size_t pupil_smem = 0;
-    DevBuf<float> tbuf;
-    PadIndex pad() const { return PadIndex{xpad.p, ypad.p, footprint.p, kx, ky, maxnx, maxny}; }
+    DevBuf<int2> vrow;
+    // k_hxt_rows: layer rows per thread, CTAs per instance, the transposed lists as windows
+    int hrows = 0, nblk_hxt = 0;
+    DevBuf<int> hxt_x0, hxt_y0;
+    DevBuf<float> hxt_xw, hxt_yw;
+    HxtTab hxttab{};
+    // the back-projected OPD between the two: [b][w][orows][ostride], zero beyond the pupil
+    DevBuf<float> obuf;
+    int orows = 0, ostride = 0;
     DevBuf<LayerDev> lay;
     std::vector<LayerDev> lay_h;
     LayerTab laytab{};  // lay_h by value, for kernel parameters
@@ -263,8 +266,18 @@ struct Recon {
     // ------------------------------------------------------------------
     void build(const mb_recon_desc *d);
     void build_hx_tables(const mb_recon_desc *d);
-    void build_pad(int min_kx = 1, int min_ky = 1);
+    void build_blocking();
+    int pupil_vrows(int rows, std::vector<int2> *out = nullptr) const;
+    size_t pupil_smem_of(int rows) const;
+    int max_pos() const {
+        int m = 1;
+        for (const WfsDev &w : wfs_h) m = std::max(m, w.pos);
+        return m;
+    }
     void set_pupil_rows(int rows);
+    int hxt_window(int l, int rows) const;
+    int hxt_blocks(int rows) const;
+    void set_hxt_rows(int rows);
     void rebuild_fdpcg_device();
     int autotune(int reps, float *ms_out);
     void pupil_rows(bool from_x, const float *xin, cudaStream_t s);
@@ -272,7 +285,6 @@ struct Recon {
     // the arguments of those launches (also gathered by a ReconGroup)
     PupilArgs pupil_args(bool from_x, const float *xin, int w0) const;
     HxtArgs hxt_args(const float *xin, float *out, double *dot_part, int do_l2, int k) const;
-    int hxt_ni() const { return nb > 1 ? 2 : 1; }
     void build_wfs_tables(const mb_recon_desc *d);
     void build_fdpcg(const mb_fdpcg_desc *fd);
     void build_fit(const mb_fit_desc *f);
@@ -425,6 +437,7 @@ static void build_ray_tables(const mb_grid &og, int ndir, int nt, const mb_grid 
     rt.h_ptr = std::move(ptr);
     rt.h_idxptr = std::move(idxptr);
     rt.h_ent = std::move(ent);
+    rt.h_fwd = std::move(tab);
 }
 
 void Recon::build_hx_tables(const mb_recon_desc *d) {
@@ -439,111 +452,228 @@ void Recon::build_hx_tables(const mb_recon_desc *d) {
                      false, hx);
 }
 
-// Fixed-width copies of the transposed x and y lists of every (WFS, layer),
-// padded with (index 0, weight 0) after the real entries (at least min_kx /
-// min_ky wide: a ReconGroup gives its members one width, and the padding
-// adds exact zeros), and the pupil-row blocking of k_pupil_rows.
-void Recon::build_pad(int min_kx, int min_ky) {
-    maxnx = maxny = 0;
-    for (int l = 0; l < nps; l++) {
-        maxnx = std::max(maxnx, lay_h[l].nx);
-        maxny = std::max(maxny, lay_h[l].ny);
-    }
-    kx = std::max(1, min_kx);
-    ky = std::max(1, min_ky);
-    for (int w = 0; w < nwfs; w++)
-        for (int l = 0; l < nps; l++)
-            for (int axis = 0; axis < 2; axis++) {
-                const int tb = hx.h_ptr[(w * nps + l) * 2 + axis];
-                const int n = axis ? lay_h[l].ny : lay_h[l].nx;
-                int &K = axis ? ky : kx;
-                for (int j = 0; j < n; j++) K = std::max(K, hx.h_idxptr[tb + j + 1] - hx.h_idxptr[tb + j]);
-            }
+constexpr size_t kMaxRowSmem = 200 * 1024;  // dynamic shared memory of a row block
+
+// The row blocking of k_pupil_rows and k_hxt_rows.
+void Recon::build_blocking() {
     MB_REQUIRE(nps <= kMaxLayers, "at most %d reconstructed layers (%d)", kMaxLayers, nps);
-    MB_REQUIRE(kx <= kMaxPadX, "transposed x lists wider than %d (%d)", kMaxPadX, kx);
-    MB_REQUIRE(ky <= kMaxPadY, "transposed y lists wider than %d (%d)", kMaxPadY, ky);
-    MB_REQUIRE(nxp <= kThreads, "pupil grid wider than %d (%d)", kThreads, nxp);
-    std::vector<GatherW> xp((size_t)nwfs * ncols * kx, GatherW{0, 0.f});
-    std::vector<GatherW> yp((size_t)nwfs * nps * maxny * ky, GatherW{0, 0.f});
     for (int w = 0; w < nwfs; w++)
         for (int l = 0; l < nps; l++)
             for (int axis = 0; axis < 2; axis++) {
                 const int tb = hx.h_ptr[(w * nps + l) * 2 + axis];
                 const int n = axis ? lay_h[l].ny : lay_h[l].nx;
-                for (int j = 0; j < n; j++)
-                    for (int a = hx.h_idxptr[tb + j], k = 0; a < hx.h_idxptr[tb + j + 1]; a++, k++) {
-                        if (axis) yp[((size_t)(w * nps + l) * maxny + j) * ky + k] = hx.h_ent[a];
-                        else xp[((size_t)w * kx + k) * ncols + lay_h[l].tcol + j] = hx.h_ent[a];  // entry-major
-                    }
+                for (int j = 0; j < n; j++) {
+                    const int k = hx.h_idxptr[tb + j + 1] - hx.h_idxptr[tb + j];
+                    MB_REQUIRE(k <= kMaxPad, "transposed %s lists wider than %d (%d)", axis ? "y" : "x", kMaxPad, k);
+                }
             }
-    xpad.upload(xp);
-    ypad.upload(yp);
-    // footprint of every WFS on every layer: first and last+1 column and row
-    // with a non-empty transposed list
-    std::vector<int4> fp((size_t)nwfs * nps);
-    for (int w = 0; w < nwfs; w++)
-        for (int l = 0; l < nps; l++) {
-            int lo[2] = {INT32_MAX, INT32_MAX}, hi[2] = {-1, -1};
-            for (int axis = 0; axis < 2; axis++) {
-                const int tb = hx.h_ptr[(w * nps + l) * 2 + axis];
-                const int n = axis ? lay_h[l].ny : lay_h[l].nx;
-                for (int j = 0; j < n; j++)
-                    if (hx.h_idxptr[tb + j + 1] > hx.h_idxptr[tb + j]) {
-                        lo[axis] = std::min(lo[axis], j);
-                        hi[axis] = j;
-                    }
-            }
-            fp[(size_t)w * nps + l] = hi[0] < 0 || hi[1] < 0 ? make_int4(0, 0, 0, 0)
-                                                             : make_int4(lo[0], hi[0] + 1, lo[1], hi[1] + 1);
-        }
-    footprint.upload(fp);
+    MB_REQUIRE(nxp <= kThreads, "pupil grid wider than %d (%d)", kThreads, nxp);
+    ostride = std::max(nxp, kMaxPad);
+    orows = nyp;
+    for (int l = 0; l < nps; l++)
+        for (int rt : {1, 2, 4}) orows = std::max(orows, hxt_window(l, rt));
     // pupil rows per CTA: as many row blocks per WFS as one wave of 4 CTAs on
-    // each of 148 SMs holds, at least 3 and with at least 4 rows per block
-    // (the measured optimum of the 30 m system at 1, 32 and 64 instances);
-    // Recon::autotune replaces the guess by measurement.
+    // each of 148 SMs holds, at least 3 and with at least 4 rows per block;
+    // Recon::autotune replaces the guess by measurement.  Fewer rows where
+    // the block's tables would not fit.
     const long nmax = (nyp + 3) / 4;
     const long tiles = std::max(3L, std::min(nmax, (long)(4 * 148) / std::max(1L, (long)nwfs * nb)));
     int rows = (int)((nyp + tiles - 1) / tiles);
+    while (rows > 1 && pupil_smem_of(rows) > kMaxRowSmem) rows = (rows + 1) / 2;
     if (const char *e = std::getenv("MAOS_B200_PUPIL_ROWS")) {  // tuning override
         const int v = std::atoi(e);
         if (v >= 1 && v <= 64) rows = v;
     }
-    tw = (long)nyp * ncols;
     set_pupil_rows(rows);
+    // layer rows per thread of k_hxt_rows: more rows share their pupil rows,
+    // fewer give more threads: 4 from 8 CTAs per SM on, 1 below 4
+    auto threads = [&](int rt) {
+        long n = 0;
+        for (int l = 0; l < nps; l++) n += (long)((lay_h[l].ny + rt - 1) / rt) * lay_h[l].nx;
+        return n * nb;
+    };
+    set_hxt_rows(threads(4) >= 148L * 8 * kHxtThreads ? 4 : threads(2) >= 148L * 4 * kHxtThreads ? 2 : 1);
+}
+
+// The layer rows that each block of `rows` pupil rows (with its halo)
+// interpolates between: [w][tile][layer] first row, rows | their offset among
+// the block's rows << 16.  Returns the most rows of a block.
+int Recon::pupil_vrows(int rows, std::vector<int2> *out) const {
+    int most = 0;
+    const int nt = (nyp + rows - 1) / rows;
+    for (int w = 0; w < nwfs; w++) {
+        const int pos = wfs_h[w].pos;
+        for (int t = 0; t < nt; t++) {
+            const int r0 = t * rows, r1 = std::min(nyp, r0 + rows);
+            const int ca = std::max(0, r0 - pos), e = std::min(nyp - pos, r1) + pos;
+            int off = 0;
+            for (int l = 0; l < nps; l++) {
+                const AxisW *y = hx.h_fwd.data() + (size_t)(w * nps + l) * (nxp + nyp) + nxp;
+                int lo = INT32_MAX, hi = -1;
+                for (int i = ca; i < e; i++)
+                    if (y[i].k >= 0) {
+                        lo = std::min(lo, y[i].k);
+                        hi = std::max(hi, y[i].k + 1);
+                    }
+                const int n = hi < 0 ? 0 : hi + 1 - lo;
+                if (out) out->push_back(make_int2(hi < 0 ? 0 : lo, n | off << 16));
+                off += n;
+            }
+            most = std::max(most, off);
+        }
+    }
+    return most;
+}
+
+size_t Recon::pupil_smem_of(int rows) const {
+    return (size_t)pupil_rows_smem_floats(rows, nxp, nps, pupil_vrows(rows), max_pos()) * sizeof(float);
+}
+
+// Every instantiation of k_pupil_rows.
+using PupilKern = void (*)(PupilArgs);
+static PupilKern pupil_kern(bool from_x, bool p2) {
+    return from_x ? (p2 ? k_pupil_rows<true, 2> : k_pupil_rows<true, 1>)
+                  : (p2 ? k_pupil_rows<false, 2> : k_pupil_rows<false, 1>);
+}
+using PupilGroupKern = void (*)(GroupTab<PupilArgs>);
+static PupilGroupKern pupil_group_kern(bool from_x, bool p2) {
+    return from_x ? (p2 ? k_pupil_rows_group<true, 2> : k_pupil_rows_group<true, 1>)
+                  : (p2 ? k_pupil_rows_group<false, 2> : k_pupil_rows_group<false, 1>);
+}
+// and of k_hxt_rows, by the layer rows per thread
+using HxtKern = void (*)(HxtArgs);
+static HxtKern hxt_kern(int rt) { return rt == 4 ? k_hxt_rows<4> : rt == 2 ? k_hxt_rows<2> : k_hxt_rows<1>; }
+using HxtGroupKern = void (*)(GroupTab<HxtArgs>);
+static HxtGroupKern hxt_group_kern(int rt) {
+    return rt == 4 ? k_hxt_rows_group<4> : rt == 2 ? k_hxt_rows_group<2> : k_hxt_rows_group<1>;
+}
+// Allow `smem` bytes of dynamic shared memory; the largest any caller asked
+// for stays allowed (kernels are shared by all reconstructors).
+template <class K>
+static void allow_smem(K kern, size_t smem) {
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lk(mu);
+    cudaFuncAttributes a;
+    MB_CUDA_TRY(cudaFuncGetAttributes(&a, (const void *)kern));
+    if ((size_t)a.maxDynamicSharedSizeBytes < smem)
+        MB_CUDA_TRY(cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 }
 
 void Recon::set_pupil_rows(int rows) {
-    const size_t sm = (size_t)pupil_rows_smem_floats(rows, nxp, nps, ncols, kx) * sizeof(float);
-    MB_REQUIRE(sm <= 200 * 1024, "pupil row block needs %zu bytes of shared memory", sm);
+    std::vector<int2> v;
+    pvrows = pupil_vrows(rows, &v);
+    const size_t sm = (size_t)pupil_rows_smem_floats(rows, nxp, nps, pvrows, max_pos()) * sizeof(float);
+    MB_REQUIRE(sm <= kMaxRowSmem, "pupil row block needs %zu bytes of shared memory", sm);
+    vrow.upload(v);
     prows = rows;
     ptiles = (nyp + prows - 1) / prows;
     pupil_smem = sm;
-    for (auto k : {k_pupil_rows<true, 1, 8>, k_pupil_rows<true, 2, 8>, k_pupil_rows<false, 1, 8>,
-                   k_pupil_rows<false, 2, 8>, k_pupil_rows<true, 1, 16>, k_pupil_rows<true, 2, 16>,
-                   k_pupil_rows<false, 1, 16>, k_pupil_rows<false, 2, 16>})
-        MB_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pupil_smem));
+    for (bool fx : {false, true})
+        for (bool p2 : {false, true}) allow_smem(pupil_kern(fx, p2), pupil_smem);
+}
+
+int Recon::hxt_blocks(int rows) const {
+    int n = 0;
+    for (int l = 0; l < nps; l++) n += (int)nblocks((long)((lay_h[l].ny + rows - 1) / rows) * lay_h[l].nx, kHxtThreads);
+    return n;
+}
+
+// The first and one past the last real entry (weight not 0) of list j of (w, l, axis).
+static void list_span(const RayTables &hx, int w, int l, int nps, int axis, int j, int &lo, int &hi) {
+    const int tb = hx.h_ptr[(w * nps + l) * 2 + axis];
+    for (int a = hx.h_idxptr[tb + j]; a < hx.h_idxptr[tb + j + 1]; a++)
+        if (hx.h_ent[a].w != 0.f) {
+            lo = std::min(lo, hx.h_ent[a].i);
+            hi = std::max(hi, hx.h_ent[a].i + 1);
+        }
+}
+
+static int hxt_width(int k) { return k <= 2 ? 2 : k <= 4 ? k : k <= 6 ? 6 : 8; }
+
+// Pupil rows of the widest row window of a layer, in whole chunks.
+int Recon::hxt_window(int l, int rows) const {
+    int kx = 1, ky = 1;
+    for (int w = 0; w < nwfs; w++) {
+        for (int j = 0; j < lay_h[l].nx; j++) {
+            int lo = INT32_MAX, hi = -1;
+            list_span(hx, w, l, nps, 0, j, lo, hi);
+            if (hi > 0) kx = std::max(kx, hi - lo);
+        }
+        for (int j0 = 0; j0 < lay_h[l].ny; j0 += rows) {
+            int lo = INT32_MAX, hi = -1;
+            for (int j = j0; j < std::min(lay_h[l].ny, j0 + rows); j++) list_span(hx, w, l, nps, 1, j, lo, hi);
+            if (hi > 0) ky = std::max(ky, hi - lo);
+        }
+    }
+    const int c = hxt_chunk(hxt_width(kx));
+    return (ky + c - 1) / c * c;
+}
+
+// The transposed lists of every (layer, WFS) as windows for `rows` layer rows
+// per thread: a list's (a row group's) real entries are consecutive pupil
+// columns (rows); the window starts there, or earlier where it would leave the
+// buffer, with zero weights around the real entries.
+void Recon::set_hxt_rows(int rows) {
+    std::vector<int> x0, y0;
+    std::vector<float> xw, yw;
+    HxtTab tab{};
+    for (int l = 0; l < nps; l++) {
+        HxtLayer &H = tab.l[l];
+        const int nx = lay_h[l].nx, ny = lay_h[l].ny;
+        int k = 1;
+        for (int w = 0; w < nwfs; w++)
+            for (int j = 0; j < nx; j++) {
+                int lo = INT32_MAX, hi = -1;
+                list_span(hx, w, l, nps, 0, j, lo, hi);
+                if (hi > 0) k = std::max(k, hi - lo);
+            }
+        H.k = hxt_width(k);
+        H.n = hxt_window(l, rows);
+        H.groups = (ny + rows - 1) / rows;
+        H.blocks = (int)nblocks((long)H.groups * nx, kHxtThreads);
+        H.xoff = (int)x0.size();
+        H.roff = (int)y0.size();
+        H.woff = (int)(yw.size() / rows);
+        for (int w = 0; w < nwfs; w++) {
+            const size_t xb = xw.size(), tx = hx.h_ptr[(w * nps + l) * 2], ty = hx.h_ptr[(w * nps + l) * 2 + 1];
+            xw.resize(xb + (size_t)kMaxPad * nx, 0.f);
+            for (int j = 0; j < nx; j++) {
+                int lo = INT32_MAX, hi = -1;
+                list_span(hx, w, l, nps, 0, j, lo, hi);
+                const int at = hi < 0 ? -1 : std::max(0, std::min(lo, ostride - H.k));
+                x0.push_back(at);
+                if (hi < 0) continue;
+                for (int a = hx.h_idxptr[tx + j]; a < hx.h_idxptr[tx + j + 1]; a++)
+                    if (hx.h_ent[a].w != 0.f) xw[xb + (size_t)(hx.h_ent[a].i - at) * nx + j] = hx.h_ent[a].w;
+            }
+            for (int g = 0; g < H.groups; g++) {
+                int lo = INT32_MAX, hi = -1;
+                const int j1 = std::min(ny, (g + 1) * rows);
+                for (int j = g * rows; j < j1; j++) list_span(hx, w, l, nps, 1, j, lo, hi);
+                const int at = hi < 0 ? -1 : std::max(0, std::min(lo, orows - H.n));
+                y0.push_back(at);
+                const size_t yb = yw.size();
+                yw.resize(yb + (size_t)H.n * rows, 0.f);
+                if (hi < 0) continue;
+                for (int j = g * rows; j < j1; j++)
+                    for (int a = hx.h_idxptr[ty + j]; a < hx.h_idxptr[ty + j + 1]; a++)
+                        if (hx.h_ent[a].w != 0.f)
+                            yw[yb + (size_t)(hx.h_ent[a].i - at) * rows + (j - g * rows)] = hx.h_ent[a].w;
+            }
+        }
+    }
+    hxt_x0.upload(x0);
+    hxt_y0.upload(y0);
+    hxt_xw.upload(xw);
+    hxt_yw.upload(yw);
+    hxttab = tab;
+    hrows = rows;
+    nblk_hxt = hxt_blocks(rows);
 }
 
 PupilArgs Recon::pupil_args(bool from_x, const float *xin, int w0) const {
-    return PupilArgs{xin,    grad.p, tt.p,   tbuf.p, hx.fwd.p, laytab, wfstab, pad(), w0,    nps, nwfs, nxp,
-                     nyp,    nxtot,  ngrad,  tw,     ncols,    prows,  from_x ? 0 : 1, act()};
-}
-
-// The k_pupil_rows instantiation for a subaperture/pupil ratio and layer count.
-using PupilKern = void (*)(const float *, const float *, const float *, float *, const AxisW *, LayerTab, WfsTab,
-                           PadIndex, int, int, int, int, int, long, long, long, int, int, int, const int *);
-static PupilKern pupil_kern(bool from_x, bool p2, bool few) {
-    return from_x ? (p2 ? (few ? k_pupil_rows<true, 2, 8> : k_pupil_rows<true, 2, 16>)
-                        : (few ? k_pupil_rows<true, 1, 8> : k_pupil_rows<true, 1, 16>))
-                  : (p2 ? (few ? k_pupil_rows<false, 2, 8> : k_pupil_rows<false, 2, 16>)
-                        : (few ? k_pupil_rows<false, 1, 8> : k_pupil_rows<false, 1, 16>));
-}
-using PupilGroupKern = void (*)(GroupTab<PupilArgs>);
-static PupilGroupKern pupil_group_kern(bool from_x, bool p2, bool few) {
-    return from_x ? (p2 ? (few ? k_pupil_rows_group<true, 2, 8> : k_pupil_rows_group<true, 2, 16>)
-                        : (few ? k_pupil_rows_group<true, 1, 8> : k_pupil_rows_group<true, 1, 16>))
-                  : (p2 ? (few ? k_pupil_rows_group<false, 2, 8> : k_pupil_rows_group<false, 2, 16>)
-                        : (few ? k_pupil_rows_group<false, 1, 8> : k_pupil_rows_group<false, 1, 16>));
+    return PupilArgs{xin,  grad.p, tt.p,  obuf.p, hx.fwd.p, vrow.p, laytab,  wfstab,         w0,   nps, nwfs, nxp,
+                     nyp,  nxtot,  ngrad, prows,  ptiles,   pvrows, ostride, orows * ostride, from_x ? 0 : 1, act()};
 }
 
 // Launch k_pupil_rows over every WFS: one launch per run of consecutive WFS
@@ -552,45 +682,21 @@ void Recon::pupil_rows(bool from_x, const float *xin, cudaStream_t s) {
     for (int w0 = 0; w0 < nwfs;) {
         int w1 = w0 + 1;
         while (w1 < nwfs && wfs_h[w1].pos == wfs_h[w0].pos) w1++;
-        const PupilArgs a = pupil_args(from_x, xin, w0);
-        launch(pupil_kern(from_x, wfs_h[w0].pos == 2, nps <= 8), dim3(ptiles, w1 - w0, nb), dim3(kThreads),
-               pupil_smem, s, a.x, a.grad, a.tt, a.t, a.tab, a.lt, a.wt, a.pi, a.wbase, a.nps, a.nwfs, a.nxp, a.nyp,
-               a.nxtot, a.ngrad, a.tw, a.ncols, a.rows, a.do_tt, a.act);
+        launch(pupil_kern(from_x, wfs_h[w0].pos == 2), dim3(ptiles, w1 - w0, nb), dim3(kThreads), pupil_smem, s,
+               pupil_args(from_x, xin, w0));
         w0 = w1;
     }
 }
 
 HxtArgs Recon::hxt_args(const float *xin, float *out, double *dot_part, int do_l2, int k) const {
-    return HxtArgs{tbuf.p, xin, out, dot_part, pad(), laytab, nps, nwfs, nyp, nxtot, tw, do_l2, scal(), k, nb, act()};
+    return HxtArgs{obuf.p, xin,     out,   dot_part, HxtIndex{hxt_x0.p, hxt_xw.p, hxt_y0.p, hxt_yw.p},
+                   hxttab, laytab,  nps,   nwfs,     orows,
+                   ostride, nxtot,  do_l2, scal(),   k,
+                   act()};
 }
 
-using HxtKern = void (*)(const float *, const float *, float *, double *, PadIndex, LayerTab, int, int, int, long,
-                         long, int, CgScal, int, int, const int *);
-static HxtKern hxt_kern(int ky, int ni) {
-    static const HxtKern tab1[kMaxPadY] = {k_hxt_rows<1, 1>, k_hxt_rows<2, 1>, k_hxt_rows<3, 1>, k_hxt_rows<4, 1>,
-                                           k_hxt_rows<5, 1>, k_hxt_rows<6, 1>, k_hxt_rows<7, 1>, k_hxt_rows<8, 1>};
-    static const HxtKern tab2[kMaxPadY] = {k_hxt_rows<1, 2>, k_hxt_rows<2, 2>, k_hxt_rows<3, 2>, k_hxt_rows<4, 2>,
-                                           k_hxt_rows<5, 2>, k_hxt_rows<6, 2>, k_hxt_rows<7, 2>, k_hxt_rows<8, 2>};
-    return ni == 2 ? tab2[ky - 1] : tab1[ky - 1];
-}
-using HxtGroupKern = void (*)(GroupTab<HxtArgs>);
-static HxtGroupKern hxt_group_kern(int ky, int ni) {
-    static const HxtGroupKern tab1[kMaxPadY] = {k_hxt_rows_group<1, 1>, k_hxt_rows_group<2, 1>, k_hxt_rows_group<3, 1>,
-                                                k_hxt_rows_group<4, 1>, k_hxt_rows_group<5, 1>, k_hxt_rows_group<6, 1>,
-                                                k_hxt_rows_group<7, 1>, k_hxt_rows_group<8, 1>};
-    static const HxtGroupKern tab2[kMaxPadY] = {k_hxt_rows_group<1, 2>, k_hxt_rows_group<2, 2>, k_hxt_rows_group<3, 2>,
-                                                k_hxt_rows_group<4, 2>, k_hxt_rows_group<5, 2>, k_hxt_rows_group<6, 2>,
-                                                k_hxt_rows_group<7, 2>, k_hxt_rows_group<8, 2>};
-    return ni == 2 ? tab2[ky - 1] : tab1[ky - 1];
-}
-
-// k_hxt_rows at the padded y-list width, two instances per thread when the
-// batch has more than one.
 void Recon::hxt_rows(const float *xin, float *out, double *dot_part, int do_l2, int k, cudaStream_t s) {
-    const int ni = hxt_ni();
-    const HxtArgs a = hxt_args(xin, out, dot_part, do_l2, k);
-    launch(hxt_kern(ky, ni), dim3(nblk_hxt, (nb + ni - 1) / ni), dim3(hxt_threads), 0, s, a.t, a.xin, a.out,
-           a.dot_part, a.pi, a.lt, a.nps, a.nwfs, a.nyp, a.nxtot, a.tw, a.do_l2, a.S, a.kit, a.nb, a.act);
+    launch(hxt_kern(hrows), dim3(nblk_hxt, nb), dim3(kHxtThreads), 0, s, hxt_args(xin, out, dot_part, do_l2, k));
 }
 
 void Recon::build_wfs_tables(const mb_recon_desc *d) {
@@ -1232,8 +1338,6 @@ void Recon::build(const mb_recon_desc *d) {
         lay_h[l].nx = g.nx;
         lay_h[l].ny = g.ny;
         lay_h[l].off = xoff[l];
-        lay_h[l].tcol = ncols;
-        ncols += g.nx;
         xoff[l + 1] = xoff[l] + (long)g.nx * g.ny;
     }
     nxtot = xoff[nps];
@@ -1253,20 +1357,20 @@ void Recon::build(const mb_recon_desc *d) {
     ngrad = goff[nwfs];
     set_l2c(d->l2c);
     build_hx_tables(d);
-    build_pad();
     build_wfs_tables(d);
+    build_blocking();
     nblk_x = (int)nblocks(nxtot);
-    nblk_hxt = nblk_x;
     nblk_tt = (int)nblocks(nsamax);
     nsc = maxit + 3;
     const size_t NX = (size_t)nb * nxtot;
     x.alloc(NX); r.alloc(NX); p.alloc(NX); z.alloc(NX); Ap.alloc(NX); rhs.alloc(NX);
     opd.alloc((size_t)nb * nwfs * np);
-    tbuf.alloc((size_t)nb * nwfs * tw);
+    obuf.alloc((size_t)nb * nwfs * orows * ostride);
+    obuf.zero_async(stream);
     grad.alloc((size_t)nb * ngrad);
     gin.alloc((size_t)nb * ngrad);
     tt_part.alloc((size_t)nb * nwfs * nblk_tt * 2);
-    pap_part.alloc((size_t)nb * nblocks(nxtot, 64));  // room for k_hxt_rows CTAs down to 64 threads
+    pap_part.alloc((size_t)nb * hxt_blocks(1));  // room for k_hxt_rows CTAs of any row count
     rr_part.alloc((size_t)nb * nblk_x);
     rz_part.alloc((size_t)nb * nblk_x);
     bb_part.alloc((size_t)nb * nblk_x);
@@ -1742,13 +1846,13 @@ void Recon::time_stages(int reps, float *ms, double *bytes, int *launches) {
         tab_wfs += nsa[w] * (8.0 * n1 * n1 + 12.0) + 4.0 * np;
     }
     const double nx = (double)nxtot;
-    const double trow = (double)nwfs * tw;  // row-buffer floats per instance
+    const double no = (double)nwfs * np;        // back-projected OPD per instance
     const double nbk = (double)fd_nbh * fd_bs;  // block members (spectrum bins read by k_fd_mul)
     double nh = 0;                              // half-spectrum bins per instance
     for (int l = 0; l < nps; l++) nh += (double)lay_h[l].ny * (lay_h[l].nx / 2 + 1);
     const double by[8] = {
-        B * (F * nx + F * trow) + (double)hx.fwd.n * sizeof(AxisW) + tab_wfs + (double)xpad.n * sizeof(GatherW),
-        B * (F * trow + 2 * F * nx) + (double)ypad.n * sizeof(GatherW),       // t, p -> Ap
+        B * (F * nx + F * no) + (double)hx.fwd.n * sizeof(AxisW) + tab_wfs,   // p -> o
+        B * (F * no + 2 * F * nx) + 4.0 * (hxt_xw.n + hxt_yw.n),  // o, p -> Ap
         B * (6 * F * nx),                                                    // x,r,p,Ap read; x,r written
         B * (3 * F * nx),                                                    // p,z read; p written
         B * (6 * F * nx + 8.0 * nh),                          // x,r,p,Ap read; x,r written; spectrum written
@@ -1841,7 +1945,7 @@ int Recon::autotune(int reps, float *ms_out) {
     float tbest = 1e30f;
     for (size_t c = 0; c < cand.size(); c++) {
         if (ms_out && c < 3) ms_out[c] = -1.f;
-        if ((size_t)pupil_rows_smem_floats(cand[c], nxp, nps, ncols, kx) * sizeof(float) > 200 * 1024) continue;
+        if (pupil_smem_of(cand[c]) > kMaxRowSmem) continue;
         set_pupil_rows(cand[c]);
         op_lhs(p.p, Ap.p, nullptr, stream);  // warm
         MB_CUDA_TRY(cudaEventRecord(e0, stream));
@@ -1858,14 +1962,12 @@ int Recon::autotune(int reps, float *ms_out) {
         }
     }
     set_pupil_rows(best);
-    // k_hxt_rows's CTA size: 256, 128 or 64 threads (smaller CTAs spread a
-    // small batch over more SMs)
+    // k_hxt_rows's layer rows per thread
     {
-        int bt = hxt_threads;
+        int bt = hrows;
         float tb = 1e30f;
-        for (int th : {256, 128, 64}) {
-            hxt_threads = th;
-            nblk_hxt = (int)nblocks(nxtot, th);
+        for (int hr : {1, 2, 4}) {
+            set_hxt_rows(hr);
             op_lhs(p.p, Ap.p, nullptr, stream);  // warm
             MB_CUDA_TRY(cudaEventRecord(e0, stream));
             for (int i = 0; i < reps; i++) op_lhs(p.p, Ap.p, nullptr, stream);
@@ -1875,11 +1977,10 @@ int Recon::autotune(int reps, float *ms_out) {
             MB_CUDA_TRY(cudaEventElapsedTime(&t, e0, e1));
             if (t < tb) {
                 tb = t;
-                bt = th;
+                bt = hr;
             }
         }
-        hxt_threads = bt;
-        nblk_hxt = (int)nblocks(nxtot, bt);
+        set_hxt_rows(bt);
     }
     capture_graph();
     // the preconditioner's form: three kernels, or one fused cluster kernel,
@@ -2063,7 +2164,7 @@ struct ReconGroup {
         }
     }
     // k_pupil_rows of the listed members in as few launches as their
-    // subaperture/pupil ratios and layer counts allow (one for the presets)
+    // subaperture/pupil ratios allow
     void pupil_rows(bool from_x, const std::vector<int> &who, const std::vector<const float *> &xin,
                     cudaStream_t s) {
         struct E {
@@ -2080,11 +2181,11 @@ struct ReconGroup {
                 while (w1 < R.nwfs && R.wfs_h[w1].pos == R.wfs_h[w0].pos) w1++;
                 es.push_back(E{R.pupil_args(from_x, xin[i], w0),
                                make_uint3((unsigned)R.ptiles, (unsigned)(w1 - w0), (unsigned)R.nb),
-                               (R.wfs_h[w0].pos == 2 ? 2 : 0) + (R.nps <= 8 ? 1 : 0), R.pupil_smem});
+                               R.wfs_h[w0].pos == 2 ? 1 : 0, R.pupil_smem});
                 w0 = w1;
             }
         }
-        for (int key = 0; key < 4; key++) {
+        for (int key = 0; key < 2; key++) {
             std::vector<const E *> b;
             for (const E &e : es)
                 if (e.key == key) b.push_back(&e);
@@ -2100,19 +2201,16 @@ struct ReconGroup {
                     g.grid[e] = x.grid;
                     g.start[e + 1] = g.start[e] + x.grid.x * x.grid.y * x.grid.z;
                 }
-                launch(pupil_group_kern(from_x, key & 2, key & 1), dim3(g.start[g.n]), dim3(kThreads), pupil_smem, s,
-                       g);
+                launch(pupil_group_kern(from_x, key), dim3(g.start[g.n]), dim3(kThreads), pupil_smem, s, g);
             }
         }
     }
     void hxt_rows(const std::vector<int> &who, const std::vector<const float *> &xin, const std::vector<float *> &out,
                   const std::vector<double *> &dot, int do_l2, int k, cudaStream_t s) {
-        int ni = 1;
-        for (int i : who) ni = std::max(ni, m[i]->hxt_ni());
-        for (int ky = 1; ky <= kMaxPadY; ky++) {
+        for (int rt : {1, 2, 4}) {
             std::vector<int> b;
             for (int i : who)
-                if (m[i]->ky == ky) b.push_back(i);
+                if (m[i]->hrows == rt) b.push_back(i);
             for (size_t c0 = 0; c0 < b.size(); c0 += kMaxGroup) {
                 GroupTab<HxtArgs> g{};
                 g.n = (int)std::min(b.size() - c0, (size_t)kMaxGroup);
@@ -2121,10 +2219,10 @@ struct ReconGroup {
                     const int i = b[c0 + e];
                     const Recon &R = *m[i];
                     g.a[e] = R.hxt_args(xin[i], out[i], dot[i], do_l2, k);
-                    g.grid[e] = make_uint3((unsigned)R.nblk_x, (unsigned)((R.nb + ni - 1) / ni), 1u);
+                    g.grid[e] = make_uint3((unsigned)R.nblk_hxt, (unsigned)R.nb, 1u);
                     g.start[e + 1] = g.start[e] + g.grid[e].x * g.grid[e].y;
                 }
-                launch(hxt_group_kern(ky, ni), dim3(g.start[g.n]), dim3(kThreads), 0, s, g);
+                launch(hxt_group_kern(rt), dim3(g.start[g.n]), dim3(kHxtThreads), 0, s, g);
             }
         }
     }
@@ -2192,9 +2290,7 @@ struct ReconGroup {
         pupil_smem = 0;
         for (Recon *r : m) pupil_smem = std::max(pupil_smem, r->pupil_smem);
         for (bool fx : {false, true})
-            for (int key = 0; key < 4; key++)
-                MB_CUDA_TRY(cudaFuncSetAttribute(pupil_group_kern(fx, key & 2, key & 1),
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pupil_smem));
+            for (bool p2 : {false, true}) allow_smem(pupil_group_kern(fx, p2), pupil_smem);
         capture_into(stream, [&](cudaStream_t s) { enqueue(s); }, graph_kernels, graph);
         versions.clear();
         for (Recon *r : m) versions.push_back(r->graph_version);
@@ -2203,12 +2299,9 @@ struct ReconGroup {
         MB_REQUIRE(!m.empty(), "empty group");
         device = m[0]->device;
         maxit = m[0]->maxit;
-        int kx = 1, ky = 1;
         for (Recon *r : m) {
             MB_REQUIRE(r->device == device, "members on different devices (%d, %d)", device, r->device);
             MB_REQUIRE(r->maxit == maxit, "members with different CG iteration counts (%d, %d)", maxit, r->maxit);
-            kx = std::max(kx, r->kx);
-            ky = std::max(ky, r->ky);
         }
         for (size_t i = 0; i < m.size(); i++)
             for (size_t j = 0; j < i; j++) MB_REQUIRE(m[i] != m[j], "a reconstructor appears twice in the group");
@@ -2220,14 +2313,6 @@ struct ReconGroup {
             return (long)m[a]->nb * m[a]->nxtot > (long)m[b]->nb * m[b]->nxtot;
         });
         MB_CUDA_TRY(cudaSetDevice(device));
-        // one list width for all members (their own graphs are recaptured)
-        for (Recon *r : m)
-            if (r->kx != kx || r->ky != ky) {
-                const int rows = r->prows;
-                r->build_pad(kx, ky);
-                r->set_pupil_rows(rows);
-                r->capture_graph();
-            }
         MB_CUDA_TRY(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
         MB_CUDA_TRY(cudaEventCreateWithFlags(&fork_ev, cudaEventDisableTiming));
         for (size_t i = 0; i < m.size(); i++) {

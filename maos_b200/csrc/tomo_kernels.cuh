@@ -8,9 +8,8 @@
 // Reference counterparts (cuda/tomo.cu, cuda/prop_wrap.cu, cuda/pcg.cu):
 //   k_hx          gpu_map2map_do forward (prop_wrap.cu:35)    -- bilinear gather
 //   k_gp          gpu_gp_do (tomo.cu:362)                     -- GP stencil + TT sums
-//   k_pupil_rows  gpu_map2map_do + gpu_gp_do + gpu_gpt_do (tomo.cu:485) + the x half
-//                 of gpu_map2map_do 't', fused per block of pupil rows
-//   k_hxt_rows    y half of gpu_map2map_do 't' + gpu_laplacian_do (tomo.cu:317)
+//   k_pupil_rows  gpu_map2map_do + gpu_gp_do + gpu_gpt_do (tomo.cu:485), fused per block of pupil rows
+//   k_hxt_rows    gpu_map2map_do 't' + gpu_laplacian_do (tomo.cu:317), per block of layer rows
 //   k_fit_hxt     gpu_map2map_do 't' in gather form (DM fit)  -- no atomics
 //   k_fd_*        cufdpcg_t::P (fdpcg.cu:168)                 -- own FFTs, half spectrum
 //   k_cg_*        gpu_pcg scalar kernels (pcg.cu:27-57)       -- FP64 scalars
@@ -51,7 +50,6 @@ struct LayerDev {
     int nx, ny;
     long off;       // offset inside one instance
     float l2c;      // biharmonic weight
-    int tcol;       // first column of this layer in the row buffer of the separable Hx^T
 };
 
 constexpr int kMaxLayers = 16;  // most reconstructed layers (the Hx gather unrolls 8 or 16)
@@ -363,19 +361,30 @@ k_fit_hxt(const float *__restrict__ opd2, const float *__restrict__ xin, float *
 // ---------------------------------------------------------------------------
 // Tomography normal-equation operator in two kernels.
 //
-// The bilinear transpose Hx^T is separable: for WFS w and layer l,
-//   (Hx^T o)[jy][jx] = sum_{iy in Y(jy)} wy * sum_{ix in X(jx)} wx * o[iy][ix].
 // k_pupil_rows works on a block of pupil rows of one (instance, WFS): it
 // forms the pupil OPD (Hx, with a halo of `pos` rows), the NEA-weighted
-// gradients (GP, NEA) and GP^T of them entirely in shared memory, then
-// applies the x half of every layer's transpose and writes the partial
-// sums t[w][l][iy][jx] (coalesced).  k_hxt_rows then finishes each layer
-// point with the y half over all WFS, adds L2^T L2 x and the p.Ap partial.
-// The transposed lists are stored with a fixed width (padding: weight 0 on
-// pupil index 0), in the same order as the CSR lists, so the sums are the
-// exact adjoint of Hx and independent of the tiling.  Only the footprint of
-// each WFS on each layer (the columns and rows whose lists are not empty) is
-// computed and read; outside it every term is an exact zero.
+// gradients (GP, NEA) and GP^T of them entirely in shared memory and writes
+// the back-projected OPD o[b][w][iy][ix] (coalesced).  k_hxt_rows applies the
+// bilinear transpose to it, a block of rows of one layer per CTA, and adds
+// L2^T L2 x and the p.Ap partial.
+//
+// Both ray tracings are separable and are evaluated as such:
+//   Hx     v_l[k][ix] = sum over two layer columns, for each layer row k the
+//          block's pupil rows touch; then opd[iy][ix] = sum over two of them.
+//   Hx^T   t = sum_{ix in X(jx)} wx o[iy][ix], for each pupil row iy that
+//          reaches a thread's layer rows; then sum_{iy in Y(jy)} wy t.
+// so a value costs two (a list's) loads once per row instead of once per
+// point, and what passes between the kernels is the OPD on the pupil (6 x 63 x
+// 63 floats of a 30 m instance), not the x half on every layer's columns (6 x
+// 63 x 384 floats).  The sums run in the order of the transposed CSR lists, so
+// they are the exact adjoint of Hx and independent of the tiling.  Only the
+// footprint of each WFS on each layer (the columns and rows whose lists are
+// not empty) is computed and read; outside it every term is an exact zero.
+// Both kernels are bound by instruction issue and latency, not by bytes (L2 5%
+// of peak).  256 instances of the 30 m system: k_pupil_rows 227 -> 117 us with
+// the row-wise Hx, the contributions of GP^T kept instead of its stencils read
+// again, and no x half of Hx^T; k_hxt_rows 223 -> 113 us from column windows
+// (a row block per CTA with t in shared memory took 286).
 // ---------------------------------------------------------------------------
 // Asynchronous 4-byte global -> shared copies (cp.async): a CTA issues all of
 // a table's words at once and waits once, instead of one round trip per
@@ -391,33 +400,16 @@ __device__ __forceinline__ void cp_async_words(void *dst, const void *src, int n
         cp_async_word(static_cast<float *>(dst) + i, static_cast<const float *>(src) + i);
 }
 
-struct PadIndex {
-    const GatherW *x;   // [(w*kx + e)*ncols + tcol_l + jx]   (per WFS, entry-major over all layers' columns)
-    const GatherW *y;   // [((w*nps + l)*maxny + jy)*ky + e]
-    const int4 *fp;     // [w*nps + l]: footprint of the WFS on the layer: columns [x, y), rows [z, w)
-    int kx, ky, maxnx, maxny;
-};
+constexpr int kMaxPad = 8;      // widest transposed list
+constexpr int kPupLay = 6;      // layers whose table entries and rows k_pupil_rows loads together
 
-constexpr int kMaxPadX = 8;     // widest x list
-constexpr int kMaxPadY = 8;     // widest y list (k_hxt_rows is instantiated up to this)
-constexpr int kHxtWfs = 6;      // WFS whose gathers k_hxt_rows issues together for one instance
-
-// Dynamic shared memory of k_pupil_rows, in floats, for `rows` output rows.
-__host__ __device__ constexpr int pupil_rows_smem_floats(int rows, int nxp, int nps, int ncols, int kx) {
-    return nxp * (3 * (rows + 2) + rows + (rows + 4))      // wg, sid, opd2, opd
-           + 3 * nps * (nxp + rows + 4)                     // staged Hx axis tables
-           + 2 * ncols * kx;                                // staged x lists of the WFS
+// Dynamic shared memory of k_pupil_rows, in floats, for `rows` output rows
+// that touch at most `vrows` layer rows over all layers.
+__host__ __device__ constexpr int pupil_rows_smem_floats(int rows, int nxp, int nps, int vrows, int pos) {
+    const int c = (pos + 1) * (pos + 1) * (rows + 2), u = vrows > c ? vrows : c;
+    return 4 * nps * (rows + 4) + u * nxp + nxp * ((rows + 2) + (rows + 4));
 }
 
-// grid: (ceil(nyp/rows), nw, nb), WFS w = wbase + blockIdx.y, all with
-// subaperture/pupil ratio POS; ML >= nps bounds the unrolled layer loop.  FROM_X: the operator input is the layer
-// vector x (Hx, GP in shared memory; no tip/tilt term).  Otherwise the input
-// is a gradient vector already in `grad` (right-hand side, or the LHS with
-// the tip/tilt projection), with -PTT g per WFS in `tt` when do_tt.
-// Thread layout: each thread owns one pupil column (and a phase of the rows)
-// for the pupil-grid stages and whole layer columns for the x half of Hx^T,
-// so per-item index arithmetic is a few adds; index tables are staged in
-// shared memory and a pupil point's layer taps are issued together.
 // Grouped launches: one grid over the blocks of several reconstructors of
 // different geometries (uneven instances advanced by one launch of an
 // operator).  Entry e covers flat blocks [start[e], start[e+1]) with its own
@@ -444,117 +436,145 @@ __device__ __forceinline__ int group_entry(const GroupTab<A> &g, uint3 &bid) {
 // Arguments of one k_pupil_rows launch.
 struct PupilArgs {
     const float *x, *grad, *tt;
-    float *t;
+    float *o;              // [b][w] planes of oplane floats, rows of ostride
     const AxisW *tab;
+    const int2 *vrow;      // [(w*tiles + tile)*nps + l]: first layer row, rows | first of them in v << 16
     LayerTab lt;
     WfsTab wt;
-    PadIndex pi;
     int wbase, nps, nwfs, nxp, nyp;
-    long nxtot, ngrad, tw;
-    int ncols, rows, do_tt;
+    long nxtot, ngrad;
+    int rows, tiles, vrows, ostride, oplane, do_tt;
     const int *act;
 };
 
-// The body takes its block index as `bid` (blockIdx, or a block of one
-// member of a grouped launch, k_pupil_rows_group).
-template <bool FROM_X, int POS, int ML>
-__device__ __forceinline__ void
-pupil_rows_body(const uint3 bid, const float *__restrict__ x, const float *__restrict__ grad,
-                const float *__restrict__ tt, float *__restrict__ t, const AxisW *__restrict__ tab,
-                const LayerTab &lt, const WfsTab &wt, const PadIndex &pi, int wbase, int nps, int nwfs, int nxp,
-                int nyp, long nxtot, long ngrad, long tw, int ncols, int rows, int do_tt,
-                const int *__restrict__ act) {
+// grid: (tiles, nw, nb), WFS w = wbase + blockIdx.y, all with
+// subaperture/pupil ratio POS.  FROM_X: the operator input is the layer
+// vector x (Hx, GP in shared memory; no tip/tilt term).  Otherwise the input
+// is a gradient vector already in `grad` (right-hand side, or the LHS with
+// the tip/tilt projection), with -PTT g per WFS in `tt` when do_tt.
+// Thread layout: each thread owns one pupil column and a phase of the rows,
+// so per-item index arithmetic is a few adds.  The body takes its block index
+// as `bid` (blockIdx, or a block of one member of a grouped launch,
+// k_pupil_rows_group).
+template <bool FROM_X, int POS>
+__device__ __forceinline__ void pupil_rows_body(const uint3 bid, const PupilArgs &A) {
     pdl_enter();
     constexpr int N1 = POS + 1;
-    const int w = wbase + bid.y, b = bid.z;
-    if (inactive(act, b)) return;
-    extern __shared__ float sm[];
-    __shared__ int s_lnx[kMaxLayers], s_tcol[kMaxLayers + 1];
-    __shared__ long s_loff[kMaxLayers];
-    __shared__ int4 s_fp[kMaxLayers];
-    const WfsDev &W = wt.w[w];
+    const int w = A.wbase + bid.y, b = bid.z;
+    if (inactive(A.act, b)) return;
+    extern __shared__ float4 sm4[];
+    const WfsDev &W = A.wt.w[w];
+    const int rows = A.rows, nxp = A.nxp, nyp = A.nyp, nps = A.nps;
     const int r0 = bid.x * rows;
     const int r1 = min(nyp, r0 + rows);      // output pupil rows [r0, r1)
     const int ca = max(0, r0 - POS);         // subaperture corner rows [ca, cb)
     const int cb = min(nyp - POS, r1);
     const int nh = cb + POS - ca;            // pupil rows of the Hx halo block
-    const int cr = rows + 2;
-    const int ts = nxp + rows + 4;           // staged axis entries per layer
-    float2 *s_wg = reinterpret_cast<float2 *>(sm);                  // [cr][nxp]
-    int *s_sid = reinterpret_cast<int *>(sm + 2 * cr * nxp);         // [cr][nxp]
-    float *s_opd2 = sm + 3 * cr * nxp;                               // [rows][nxp]
-    float *s_opd = s_opd2 + rows * nxp;                              // [rows+4][nxp]
-    AxisW *s_tab = reinterpret_cast<AxisW *>(s_opd + (rows + 4) * nxp);  // [nps][ts]
-    GatherW *s_xp = reinterpret_cast<GatherW *>(reinterpret_cast<float *>(s_tab) + 3 * nps * ts);
+    const int cr = rows + 2, ts = rows + 4;
+    float4 *s_ty = sm4;                                              // [nps][ts]: row in v, its two weights
+    float *s_v = reinterpret_cast<float *>(s_ty + nps * ts);         // [vrows][nxp], then
+    float *s_c = s_v;                                                // [N1 * N1][cr][nxp] in its place
+    int *s_sid = reinterpret_cast<int *>(s_v + max(A.vrows, N1 * N1 * cr) * nxp);  // [cr][nxp]
+    float *s_opd = reinterpret_cast<float *>(s_sid + cr * nxp);      // [rows+4][nxp]
     const int nph = blockDim.x / nxp;        // row phases (nxp <= blockDim)
     const int ph = threadIdx.x / nxp, ix = threadIdx.x - ph * nxp;
     const bool colthr = ph < nph;
 
-    // stage the layer geometry and footprints, the x lists of this WFS, the
-    // subaperture map of rows [ca, cb) and, for Hx, the axis tables: all
-    // copies in flight together
-    if (threadIdx.x < nps) {
-        const LayerDev &L = lt.l[threadIdx.x];
-        s_lnx[threadIdx.x] = L.nx;
-        s_loff[threadIdx.x] = L.off;
-        s_tcol[threadIdx.x] = L.tcol;
-        s_fp[threadIdx.x] = pi.fp[w * nps + threadIdx.x];
-    }
-    if (threadIdx.x == 0) s_tcol[nps] = ncols;
-    {
-        constexpr int GW = (int)(sizeof(GatherW) / 4), AW = (int)(sizeof(AxisW) / 4);
-        cp_async_words(s_xp, pi.x + (size_t)w * ncols * pi.kx, ncols * pi.kx * GW);
-        if (cb > ca) cp_async_words(s_sid, W.samap + (size_t)ca * nxp, (cb - ca) * nxp);
-        if (FROM_X) {
-            const AxisW *tw0 = tab + (size_t)w * nps * (nxp + nyp);
-            for (int l = 0; l < nps; l++) {
-                const AxisW *tl = tw0 + (size_t)l * (nxp + nyp);
-                cp_async_words(s_tab + l * ts, tl, nxp * AW);                   // x axis
-                cp_async_words(s_tab + l * ts + nxp, tl + nxp + ca, nh * AW);   // y axis, rows [ca, ca+nh)
+    if (cb > ca) cp_async_words(s_sid, W.samap + (size_t)ca * nxp, (cb - ca) * nxp);
+    if (FROM_X) {
+        const AxisW *tw0 = A.tab + (size_t)w * nps * (nxp + nyp);
+        const int2 *vr = A.vrow + ((size_t)w * A.tiles + bid.x) * nps;
+        for (int e = threadIdx.x; e < nps * nh; e += blockDim.x) {
+            const int l = e / nh, r = e - l * nh;
+            const AxisW y = tw0[(size_t)l * (nxp + nyp) + nxp + ca + r];
+            const int2 v = vr[l];
+            s_ty[l * ts + r] = make_float4(__int_as_float(y.k < 0 ? -1 : ((v.y >> 16) + y.k - v.x) * nxp), y.w0, y.w1, 0.f);
+        }
+        // the layer rows of this block interpolated along x at the pupil columns
+        if (colthr) {
+            const float *xb = A.x + (size_t)b * A.nxtot;
+            for (int l0 = 0; l0 < nps; l0 += kPupLay) {
+                AxisW tx[kPupLay];
+                int2 v[kPupLay];
+#pragma unroll
+                for (int u = 0; u < kPupLay; u++)
+                    if (l0 + u < nps) {
+                        tx[u] = tw0[(size_t)(l0 + u) * (nxp + nyp) + ix];
+                        v[u] = vr[l0 + u];
+                    }
+#pragma unroll
+                for (int u = 0; u < kPupLay; u++) {
+                    if (l0 + u >= nps) break;
+                    const LayerDev &L = A.lt.l[l0 + u];
+                    const bool ok = tx[u].k >= 0;
+                    const float *X = xb + L.off + (size_t)v[u].x * L.nx + (ok ? tx[u].k : 0);
+                    const int n = v[u].y & 0xffff;
+                    float *d = s_v + (v[u].y >> 16) * nxp + ix;
+                    for (int j0 = ph; j0 < n; j0 += 4 * nph) {
+                        float a[4], c[4];
+#pragma unroll
+                        for (int q = 0; q < 4; q++) {
+                            const int j = j0 + q * nph;
+                            if (j < n) {
+                                a[q] = X[j * L.nx];
+                                c[q] = X[j * L.nx + 1];
+                            }
+                        }
+#pragma unroll
+                        for (int q = 0; q < 4; q++) {
+                            const int j = j0 + q * nph;
+                            if (j < n) d[j * nxp] = ok ? tx[u].w0 * a[q] + tx[u].w1 * c[q] : 0.f;
+                        }
+                    }
+                }
             }
         }
-        cp_async_wait_all();
-        __syncthreads();
     }
-    if (FROM_X) {  // Hx for pupil rows [ca, cb + POS): a point's layer taps are issued together
-        const float *xb = x + (size_t)b * nxtot;
+    cp_async_wait_all();
+    __syncthreads();
+    if (FROM_X) {  // Hx for pupil rows [ca, cb + POS): along y between two of those rows
         if (colthr)
             for (int r = ph; r < nh; r += nph) {
                 float acc = 0.f;
+                for (int l0 = 0; l0 < nps; l0 += kPupLay) {
 #pragma unroll
-                for (int l = 0; l < ML; l++) {
-                    if (l < nps) {
-                        const AxisW tx = s_tab[l * ts + ix], ty = s_tab[l * ts + nxp + r];
-                        const bool ok = tx.k >= 0 && ty.k >= 0;
-                        const int nx = s_lnx[l];
-                        const float *X = xb + s_loff[l] + (ok ? ty.k * nx + tx.k : 0);
-                        const float a = tx.w0 * X[0] + tx.w1 * X[1];
-                        const float c = tx.w0 * X[nx] + tx.w1 * X[nx + 1];
-                        if (ok) acc += ty.w0 * a + ty.w1 * c;
+                    for (int u = 0; u < kPupLay; u++) {
+                        if (l0 + u < nps) {
+                            const float4 e = s_ty[(l0 + u) * ts + r];
+                            const int k = __float_as_int(e.x);
+                            const float *v = s_v + max(k, 0) + ix;
+                            const float a = v[0], c = v[nxp];
+                            if (k >= 0) acc += e.y * a + e.z * c;
+                        }
                     }
                 }
                 s_opd[r * nxp + ix] = acc;
             }
         __syncthreads();
     }
-    {  // NEA-weighted gradients of the subapertures with corners in rows [ca, cb)
-        const float *g = FROM_X ? nullptr : grad + (size_t)b * ngrad + W.goff;
-        const bool use_tt = !FROM_X && do_tt && W.has_ptt;
-        const float ttx = use_tt ? tt[((size_t)b * nwfs + w) * 2] : 0.f;
-        const float tty = use_tt ? tt[((size_t)b * nwfs + w) * 2 + 1] : 0.f;
+    {  // NEA-weighted gradients of the subapertures with corners in rows [ca, cb), and what GP^T gives each
+       // of their stencil's points from them (plane q of s_c: the point (q / N1, q % N1) from the corner)
+        const float *g = FROM_X ? nullptr : A.grad + (size_t)b * A.ngrad + W.goff;
+        const bool use_tt = !FROM_X && A.do_tt && W.has_ptt;
+        const float ttx = use_tt ? A.tt[((size_t)b * A.nwfs + w) * 2] : 0.f;
+        const float tty = use_tt ? A.tt[((size_t)b * A.nwfs + w) * 2 + 1] : 0.f;
         if (colthr)
             for (int rr = ph; rr < cb - ca; rr += nph) {
                 const int i = rr * nxp + ix;
                 const int s = s_sid[i];  // staged subaperture map
-                if (s < 0) continue;
+                if (s < 0) {
+#pragma unroll
+                    for (int q = 0; q < N1 * N1; q++) s_c[q * cr * nxp + i] = 0.f;
+                    continue;
+                }
                 const float *ne = W.neai + 3 * s;
                 const float n0 = ne[0], n1_ = ne[1], n2 = ne[2];
+                const float2 *cf = W.gp + (size_t)s * N1 * N1;
+                float2 k[N1 * N1];
+#pragma unroll
+                for (int q = 0; q < N1 * N1; q++) k[q] = cf[q];
                 float gx = 0.f, gy = 0.f;
                 if (FROM_X) {
-                    const float2 *cf = W.gp + (size_t)s * N1 * N1;
-                    float2 k[N1 * N1];
-#pragma unroll
-                    for (int q = 0; q < N1 * N1; q++) k[q] = cf[q];
                     const float *o = s_opd + i;
 #pragma unroll
                     for (int ty = 0; ty < N1; ty++)
@@ -568,265 +588,232 @@ pupil_rows_body(const uint3 bid, const float *__restrict__ x, const float *__res
                     gx = g[s] + ttx;
                     gy = g[s + W.nsa] + tty;
                 }
-                s_wg[i] = make_float2(n0 * gx + n2 * gy, n2 * gx + n1_ * gy);
+                const float2 wg = make_float2(n0 * gx + n2 * gy, n2 * gx + n1_ * gy);
+#pragma unroll
+                for (int q = 0; q < N1 * N1; q++) s_c[q * cr * nxp + i] = k[q].x * wg.x + k[q].y * wg.y;
             }
         __syncthreads();
     }
-    if (colthr) {  // GP^T for the output rows (gather over the covering subapertures)
-        for (int pr = ph; pr < r1 - r0; pr += nph) {
-            const int py = r0 + pr;
-            float2 k[N1 * N1], v[N1 * N1];
+    if (colthr) {  // GP^T for the output rows: the contributions of the covering subapertures
+        float *ob = A.o + ((size_t)b * A.nwfs + w) * A.oplane + ix;
+        for (int py = r0 + ph; py < r1; py += nph) {
+            float acc = 0.f;
 #pragma unroll
             for (int dy = 0; dy < N1; dy++)
 #pragma unroll
                 for (int dx = 0; dx < N1; dx++) {
-                    const int cy = py - dy, cx = ix - dx;
-                    const int q = dy * N1 + dx;
-                    const bool in = cy >= ca && cy < cb && cx >= 0;
-                    const int j = in ? (cy - ca) * nxp + cx : 0;
-                    const int s = in ? s_sid[j] : -1;
-                    k[q] = s >= 0 ? W.gp[(size_t)s * N1 * N1 + q] : make_float2(0.f, 0.f);
-                    v[q] = s >= 0 ? s_wg[j] : make_float2(0.f, 0.f);
+                    const int cy = py - dy;
+                    if (cy >= ca && cy < cb && ix >= dx)
+                        acc += s_c[((dy * N1 + dx) * cr + cy - ca) * nxp + ix - dx];
                 }
-            float acc = 0.f;
-#pragma unroll
-            for (int q = 0; q < N1 * N1; q++) acc += k[q].x * v[q].x + k[q].y * v[q].y;
-            s_opd2[pr * nxp + ix] = acc;
-        }
-    }
-    __syncthreads();
-    {  // x half of Hx^T for every layer: t[w][l][iy][jx]; a thread owns whole layer columns
-        float *tb = t + (size_t)(b * nwfs + w) * tw;
-        const int kx = pi.kx, nr = r1 - r0;
-        for (int c = threadIdx.x; c < ncols; c += blockDim.x) {
-            int l = 0;
-            while (l + 1 < nps && c >= s_tcol[l + 1]) l++;
-            const int tc = s_tcol[l], lnx = s_lnx[l];
-            const int4 f = s_fp[l];
-            if (c - tc < f.x || c - tc >= f.y) continue;  // no pupil column reaches it: never read
-            GatherW e[kMaxPadX];
-#pragma unroll
-            for (int k = 0; k < kMaxPadX; k++) e[k] = k < kx ? s_xp[k * ncols + c] : GatherW{0, 0.f};  // no bank conflicts
-            float *dst = tb + (size_t)nyp * tc + (size_t)r0 * lnx + (c - tc);
-            for (int r = 0; r < nr; r++) {
-                const float *o = s_opd2 + r * nxp;
-                float sx = 0.f;
-#pragma unroll
-                for (int k = 0; k < kMaxPadX; k++)
-                    if (k < kx) sx += e[k].w * o[e[k].i];
-                dst[r * lnx] = sx;
-            }
+            ob[(size_t)py * A.ostride] = acc;
         }
     }
 }
 
-template <bool FROM_X, int POS, int ML>
-__global__ void __launch_bounds__(kThreads, 4)
-k_pupil_rows(const float *__restrict__ x, const float *__restrict__ grad, const float *__restrict__ tt,
-             float *__restrict__ t, const AxisW *__restrict__ tab, const __grid_constant__ LayerTab lt,
-             const __grid_constant__ WfsTab wt, PadIndex pi, int wbase, int nps, int nwfs, int nxp, int nyp,
-             long nxtot, long ngrad, long tw, int ncols, int rows, int do_tt,
-             const int *__restrict__ act) {
-    pupil_rows_body<FROM_X, POS, ML>(blockIdx, x, grad, tt, t, tab, lt, wt, pi, wbase, nps, nwfs, nxp, nyp, nxtot,
-                                     ngrad, tw, ncols, rows, do_tt, act);
+template <bool FROM_X, int POS>
+__global__ void __launch_bounds__(kThreads, 4) k_pupil_rows(const __grid_constant__ PupilArgs a) {
+    pupil_rows_body<FROM_X, POS>(blockIdx, a);
 }
 // grid: (sum of the entries' blocks); dynamic shared memory: the largest entry's.
-template <bool FROM_X, int POS, int ML>
-__global__ void __launch_bounds__(kThreads, 4)
-k_pupil_rows_group(const __grid_constant__ GroupTab<PupilArgs> g) {
+template <bool FROM_X, int POS>
+__global__ void __launch_bounds__(kThreads, 4) k_pupil_rows_group(const __grid_constant__ GroupTab<PupilArgs> g) {
     uint3 bid;
     const PupilArgs &a = g.a[group_entry(g, bid)];
-    pupil_rows_body<FROM_X, POS, ML>(bid, a.x, a.grad, a.tt, a.t, a.tab, a.lt, a.wt, a.pi, a.wbase, a.nps, a.nwfs,
-                                     a.nxp, a.nyp, a.nxtot, a.ngrad, a.tw, a.ncols, a.rows, a.do_tt, a.act);
+    pupil_rows_body<FROM_X, POS>(bid, a);
 }
 
-// y half of Hx^T over all WFS, + L2^T L2 x and p.Ap partials (last block:
-// alpha).  One thread per layer point and NI instances (the index work, the
-// footprint tests and the list entries are shared by the instances, and each
-// dependent step issues NI times the independent loads; the NI block sums
-// and last-block arrivals are taken together);
-// grid: (ceil(nxtot/256), ceil(nb/NI)).  KY is the padded y-list width.
-// The body takes its block index `bid` and the x extent of its grid `gx`.
-template <int KY, int NI>
-__device__ __forceinline__ void
-hxt_rows_body(const uint3 bid, const unsigned gx, const float *__restrict__ t, const float *__restrict__ xin,
-              float *__restrict__ out, double *__restrict__ dot_part, const PadIndex &pi, const LayerTab &lt,
-              int nps, int nwfs, int nyp, long nxtot, long tw, int do_l2, const CgScal &S, int kit, int nb,
-              const int *__restrict__ act) {
-    pdl_enter();
-    const int b0 = bid.y * NI;
-    bool on[NI];
-    bool any = false;
-#pragma unroll
-    for (int q = 0; q < NI; q++) {
-        on[q] = b0 + q < nb && !inactive(act, b0 + q);
-        any = any || on[q];
-    }
-    if (!any) return;
-    __shared__ double shq[NI][32];
-    __shared__ bool s_last[NI];
-    const long j = (long)bid.x * blockDim.x + threadIdx.x;
-    double dotv[NI];
-#pragma unroll
-    for (int q = 0; q < NI; q++) dotv[q] = 0;
-    if (j < nxtot) {
-        int l = 0;
-        while (l + 1 < nps && j >= lt.l[l + 1].off) l++;
-        const LayerDev L = lt.l[l];
-        const int nx = L.nx, ny = L.ny;
-        const int jj = (int)(j - L.off);
-        const int jy = jj / nx, jx = jj - jy * nx;
-        const float *tl = t + (size_t)b0 * nwfs * tw + (size_t)nyp * L.tcol + jx;
-        const size_t tinst = (size_t)nwfs * tw;  // row-buffer stride between instances
-        const GatherW *e = pi.y + ((size_t)l * pi.maxny + jy) * KY;
-        const int estep = nps * pi.maxny * KY;
-        float acc[NI];
-#pragma unroll
-        for (int q = 0; q < NI; q++) acc[q] = 0.f;
-        if constexpr (NI == 1) {
-            // one instance: the lists of kHxtWfs WFS are loaded together, then
-            // all their row-buffer values, so the WFS cost two round trips
-            // instead of two each (same sums, same order)
-            for (int w0 = 0; w0 < nwfs; w0 += kHxtWfs) {
-                GatherW ge[kHxtWfs][KY];
-                bool in[kHxtWfs];
-#pragma unroll
-                for (int u = 0; u < kHxtWfs; u++) {
-                    const int w = w0 + u;
-                    in[u] = false;
-                    if (w < nwfs) {
-                        const int4 f = pi.fp[w * nps + l];
-                        in[u] = !(jx < f.x || jx >= f.y || jy < f.z || jy >= f.w);
-                    }
-#pragma unroll
-                    for (int k = 0; k < KY; k++) ge[u][k] = in[u] ? e[(size_t)w * estep + k] : GatherW{0, 0.f};
-                }
-                float tv[kHxtWfs][KY];
-#pragma unroll
-                for (int u = 0; u < kHxtWfs; u++)
-#pragma unroll
-                    for (int k = 0; k < KY; k++)
-                        tv[u][k] = (in[u] && on[0]) ? tl[(size_t)(w0 + u) * tw + ge[u][k].i * nx] : 0.f;
-#pragma unroll
-                for (int u = 0; u < kHxtWfs; u++) {
-                    if (!in[u]) continue;
-                    float sy = 0.f;
-#pragma unroll
-                    for (int k = 0; k < KY; k++) sy += ge[u][k].w * tv[u][k];
-                    acc[0] += sy;
-                }
-            }
-        } else {
-#pragma unroll 2
-            for (int w = 0; w < nwfs; w++, e += estep, tl += tw) {
-                const int4 f = pi.fp[w * nps + l];
-                if (jx < f.x || jx >= f.y || jy < f.z || jy >= f.w) continue;  // outside this WFS's footprint
-                GatherW ge[KY];
-                float tv[NI][KY];
-#pragma unroll
-                for (int k = 0; k < KY; k++) ge[k] = e[k];
-#pragma unroll
-                for (int q = 0; q < NI; q++)
-#pragma unroll
-                    for (int k = 0; k < KY; k++) tv[q][k] = on[q] ? tl[q * tinst + ge[k].i * nx] : 0.f;
-#pragma unroll
-                for (int q = 0; q < NI; q++) {
-                    float sy = 0.f;
-#pragma unroll
-                    for (int k = 0; k < KY; k++) sy += ge[k].w * tv[q][k];
-                    acc[q] += sy;
-                }
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < NI; q++) {
-            if (!on[q]) continue;
-            const int b = b0 + q;
-            const float *X = xin ? xin + (size_t)b * nxtot + L.off : nullptr;
-            float v = acc[q];
-            if (do_l2) {  // periodic 13-point biharmonic stencil (tomo.cu gpu_laplacian_do)
-                auto wy = [&](int d) { int y = jy + d; y += (y < 0) ? ny : 0; y -= (y >= ny) ? ny : 0; return X + y * nx; };
-                auto wx = [&](int d) { int u = jx + d; u += (u < 0) ? nx : 0; u -= (u >= nx) ? nx : 0; return u; };
-                const float *Rm2 = wy(-2), *Rm1 = wy(-1), *R0 = X + jy * nx, *Rp1 = wy(1), *Rp2 = wy(2);
-                const int xm2 = wx(-2), xm1 = wx(-1), xp1 = wx(1), xp2 = wx(2);
-                const float st = 20.f * R0[jx] - 8.f * (R0[xm1] + R0[xp1] + Rm1[jx] + Rp1[jx]) +
-                                 2.f * (Rm1[xm1] + Rm1[xp1] + Rp1[xm1] + Rp1[xp1]) +
-                                 (Rm2[jx] + R0[xm2] + R0[xp2] + Rp2[jx]);
-                v += L.l2c * st;
-            }
-            out[(size_t)b * nxtot + j] = v;
-            if (dot_part && X) dotv[q] = (double)v * (double)X[jj];
-        }
-    }
-    if (dot_part) {
-        // block sums of the NI partials (the block_sum tree, NI at a time)
-        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-        for (int q = 0; q < NI; q++) {
-            const double v = warp_sum(dotv[q]);
-            if (lane == 0) shq[q][wid] = v;
-        }
-        __syncthreads();
-        if (wid == 0)
-#pragma unroll
-            for (int q = 0; q < NI; q++) {
-                double v = lane < (int)(blockDim.x >> 5) ? shq[q][lane] : 0.0;
-                v = warp_sum(v);
-                if (lane == 0 && on[q]) dot_part[(size_t)(b0 + q) * gx + bid.x] = v;
-            }
-        // last block per instance: alpha_k = (r.z)_k / (p.Ap) (cg_alpha_last, NI counters at once)
-        __threadfence();
-        __syncthreads();
-        if (threadIdx.x == 0)
-#pragma unroll
-            for (int q = 0; q < NI; q++) s_last[q] = on[q] && atomicAdd(S.cnt + b0 + q, 1u) == gx - 1;
-        __syncthreads();
-#pragma unroll
-        for (int q = 0; q < NI; q++) {
-            if (!s_last[q] || threadIdx.x >= 32) continue;
-            const int b = b0 + q;
-            const double pap = warp_sum_fresh(dot_part + (size_t)b * gx, gx);
-            if (threadIdx.x == 0) {
-                double a = S.sc[(size_t)b * S.nsc + kit] / pap;
-                if (!isfinite(a)) a = 0;  // pcg.c:80-83, pcg.cu:27-30
-                S.ab[2 * b] = (float)a;
-                S.cnt[b] = 0;
-            }
-        }
-    }
-}
+// Hx^T over all WFS, + L2^T L2 x and p.Ap partials (last block: alpha).  A
+// thread owns one layer column and RT consecutive layer rows.  For each WFS it
+// walks the pupil rows that reach them: the x half of the transpose (the
+// column's list: consecutive pupil columns, so K loads at one address) gives
+// t, and t times the row's weights to the RT layer rows (one broadcast load)
+// goes to the RT sums.  Both lists are windows of fixed width (zero weights
+// beyond the real entries), so all loads of a window are in flight together.
+constexpr int kHxtThreads = 128;
 
-template <int KY, int NI>
-__global__ void __launch_bounds__(kThreads)
-k_hxt_rows(const float *__restrict__ t, const float *__restrict__ xin, float *__restrict__ out,
-           double *__restrict__ dot_part, PadIndex pi, const __grid_constant__ LayerTab lt, int nps,
-           int nwfs, int nyp, long nxtot, long tw, int do_l2, CgScal S, int kit, int nb,
-           const int *__restrict__ act) {
-    hxt_rows_body<KY, NI>(blockIdx, gridDim.x, t, xin, out, dot_part, pi, lt, nps, nwfs, nyp, nxtot, tw, do_l2, S,
-                          kit, nb, act);
-}
+// Tables of the transpose (device), all of one layer at the layer's own width.
+struct HxtLayer {
+    int k;             // width of the column lists: 2, 3, 4, 6 or 8
+    int n;             // pupil rows of a row window (a multiple of hxt_chunk(k))
+    int xoff, roff;    // first column list, first row window (of WFS 0) of the layer
+    int woff, groups;  // first weight vector; row groups of RT rows
+    int blocks;        // CTAs of the layer
+};
+struct HxtTab {
+    HxtLayer l[kMaxLayers];
+};
+struct HxtIndex {
+    const int *x0;     // [xoff + w*nx + jx]: first pupil column, -1: no pupil column reaches it
+    const float *xw;   // [(xoff + w*nx) * 8 + e*nx + jx]: weights, entry-major
+    const int *y0;     // [roff + w*groups + g]: first pupil row, -1: none
+    const float *yw;   // [(woff + (w*groups + g)*n + i) * RT + r]: weight of pupil row y0 + i to layer row g*RT + r
+};
+__host__ __device__ constexpr int hxt_chunk(int k) { return k <= 4 ? 5 : 2; }  // pupil rows whose loads go together
+
 // Arguments of one k_hxt_rows launch.
 struct HxtArgs {
-    const float *t, *xin;
+    const float *o, *xin;
     float *out;
     double *dot_part;
-    PadIndex pi;
+    HxtIndex ix;
+    HxtTab ht;
     LayerTab lt;
-    int nps, nwfs, nyp;
-    long nxtot, tw;
+    int nps, nwfs, orows, ostride;  // rows of a WFS's plane of o, and their stride
+    long nxtot;
     int do_l2;
     CgScal S;
-    int kit, nb;
+    int kit;
     const int *act;
 };
-template <int KY, int NI>
-__global__ void __launch_bounds__(kThreads)
-k_hxt_rows_group(const __grid_constant__ GroupTab<HxtArgs> g) {
+
+template <int RT>
+__device__ __forceinline__ void load_row_weights(float (&w)[RT], const float *p) {
+    if constexpr (RT == 4) {
+        const float4 v = *reinterpret_cast<const float4 *>(p);
+        w[0] = v.x, w[1] = v.y, w[2] = v.z, w[3] = v.w;
+    } else if constexpr (RT == 2) {
+        const float2 v = *reinterpret_cast<const float2 *>(p);
+        w[0] = v.x, w[1] = v.y;
+    } else {
+#pragma unroll
+        for (int r = 0; r < RT; r++) w[r] = p[r];
+    }
+}
+
+// The transposed ray tracing of RT layer rows of column jx, over all WFS.
+template <int K, int RT>
+__device__ __forceinline__ void hxt_column(const HxtArgs &A, const HxtLayer &H, int nx, int b, int g, int jx,
+                                           float (&acc)[RT]) {
+    constexpr int C = hxt_chunk(K);
+    const int stride = A.ostride;
+    for (int w = 0; w < A.nwfs; w++) {
+        const int x0 = A.ix.x0[H.xoff + w * nx + jx];
+        const int rw = w * H.groups + g, y0 = A.ix.y0[H.roff + rw];
+        if (x0 < 0 || y0 < 0) continue;  // outside this WFS's footprint
+        float xw[K];
+        const float *xp = A.ix.xw + (size_t)(H.xoff + w * nx) * kMaxPad + jx;
+#pragma unroll
+        for (int e = 0; e < K; e++) xw[e] = xp[e * nx];
+        const float *o = A.o + ((size_t)(b * A.nwfs + w) * A.orows + y0) * stride + x0;
+        const float *yw = A.ix.yw + ((size_t)H.woff + (size_t)rw * H.n) * RT;
+        float s[RT];
+#pragma unroll
+        for (int r = 0; r < RT; r++) s[r] = 0.f;
+        for (int i = 0; i < H.n; i += C, o += C * stride, yw += C * RT) {
+            float v[C][K], wy[C][RT];
+#pragma unroll
+            for (int q = 0; q < C; q++) {
+#pragma unroll
+                for (int e = 0; e < K; e++) v[q][e] = o[q * stride + e];
+                load_row_weights<RT>(wy[q], yw + q * RT);
+            }
+#pragma unroll
+            for (int q = 0; q < C; q++) {
+                float t = 0.f;
+#pragma unroll
+                for (int e = 0; e < K; e++) t += xw[e] * v[q][e];
+#pragma unroll
+                for (int r = 0; r < RT; r++) s[r] += wy[q][r] * t;
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < RT; r++) acc[r] += s[r];
+    }
+}
+
+// grid: (blocks of all layers, nb).  The body takes its block index `bid` and
+// the x extent of its grid `gx`.
+template <int RT>
+__device__ __forceinline__ void hxt_rows_body(const uint3 bid, const unsigned gx, const HxtArgs &A) {
+    pdl_enter();
+    const int b = bid.y;
+    if (inactive(A.act, b)) return;
+    __shared__ double sh[32];
+    int l = 0, blk = bid.x;
+    while (l + 1 < A.nps && blk >= A.ht.l[l].blocks) blk -= A.ht.l[l++].blocks;
+    const LayerDev &L = A.lt.l[l];
+    const HxtLayer &H = A.ht.l[l];
+    const int nx = L.nx, ny = L.ny;
+    const int at = blk * kHxtThreads + threadIdx.x, g = at / nx, jx = at - g * nx;
+    double dotv = 0;
+    if (g < H.groups) {
+        float acc[RT];
+#pragma unroll
+        for (int r = 0; r < RT; r++) acc[r] = 0.f;
+        switch (H.k) {
+            case 2: hxt_column<2, RT>(A, H, nx, b, g, jx, acc); break;
+            case 3: hxt_column<3, RT>(A, H, nx, b, g, jx, acc); break;
+            case 4: hxt_column<4, RT>(A, H, nx, b, g, jx, acc); break;
+            case 6: hxt_column<6, RT>(A, H, nx, b, g, jx, acc); break;
+            default: hxt_column<8, RT>(A, H, nx, b, g, jx, acc); break;
+        }
+        const float *X = A.xin ? A.xin + (size_t)b * A.nxtot + L.off : nullptr;
+        float *out = A.out + (size_t)b * A.nxtot + L.off;
+        const int j0 = g * RT;
+        if (A.do_l2) {  // periodic 13-point biharmonic stencil (tomo.cu gpu_laplacian_do)
+            auto wx = [&](int d) { int u = jx + d; u += (u < 0) ? nx : 0; u -= (u >= nx) ? nx : 0; return u; };
+            const int xm2 = wx(-2), xm1 = wx(-1), xp1 = wx(1), xp2 = wx(2);
+            float c[RT + 4], m[RT + 2], p[RT + 2], f[RT], h[RT];  // the column, its neighbours at +-1 and +-2
+#pragma unroll
+            for (int q = 0; q < RT + 4; q++) {
+                int y = j0 + q - 2;
+                y += (y < 0) ? ny : 0;
+                while (y >= ny) y -= ny;  // rows past a ragged last group are not used
+                const float *R = X + y * nx;
+                c[q] = R[jx];
+                if (q >= 1 && q < RT + 3) {
+                    m[q - 1] = R[xm1];
+                    p[q - 1] = R[xp1];
+                }
+                if (q >= 2 && q < RT + 2) {
+                    f[q - 2] = R[xm2];
+                    h[q - 2] = R[xp2];
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < RT; r++) {
+                const float st = 20.f * c[r + 2] - 8.f * (m[r + 1] + p[r + 1] + c[r + 1] + c[r + 3]) +
+                                 2.f * (m[r] + p[r] + m[r + 2] + p[r + 2]) + (c[r] + f[r] + h[r] + c[r + 4]);
+                acc[r] += L.l2c * st;
+            }
+#pragma unroll
+            for (int r = 0; r < RT; r++)
+                if (j0 + r < ny) {
+                    out[(j0 + r) * nx + jx] = acc[r];
+                    if (A.dot_part) dotv += (double)acc[r] * (double)c[r + 2];
+                }
+        } else {
+#pragma unroll
+            for (int r = 0; r < RT; r++)
+                if (j0 + r < ny) out[(j0 + r) * nx + jx] = acc[r];
+        }
+    }
+    if (A.dot_part) {
+        dotv = block_sum(dotv, sh);
+        double *part = A.dot_part + (size_t)b * gx;
+        if (threadIdx.x == 0) part[bid.x] = dotv;
+        if (last_block(A.S.cnt + b, gx) && threadIdx.x < 32) {  // alpha_k = (r.z)_k / (p.Ap)
+            const double pap = warp_sum_fresh(part, gx);
+            if (threadIdx.x == 0) {
+                double a = A.S.sc[(size_t)b * A.S.nsc + A.kit] / pap;
+                if (!isfinite(a)) a = 0;  // pcg.c:80-83, pcg.cu:27-30
+                A.S.ab[2 * b] = (float)a;
+                A.S.cnt[b] = 0;
+            }
+        }
+    }
+}
+
+template <int RT>
+__global__ void __launch_bounds__(kHxtThreads) k_hxt_rows(const __grid_constant__ HxtArgs a) {
+    hxt_rows_body<RT>(blockIdx, gridDim.x, a);
+}
+template <int RT>
+__global__ void __launch_bounds__(kHxtThreads) k_hxt_rows_group(const __grid_constant__ GroupTab<HxtArgs> g) {
     uint3 bid;
     const int e = group_entry(g, bid);
-    const HxtArgs &a = g.a[e];
-    hxt_rows_body<KY, NI>(bid, g.grid[e].x, a.t, a.xin, a.out, a.dot_part, a.pi, a.lt, a.nps, a.nwfs, a.nyp, a.nxtot,
-                          a.tw, a.do_l2, a.S, a.kit, a.nb, a.act);
+    hxt_rows_body<RT>(bid, g.grid[e].x, g.a[e]);
 }
 
 // ---------------------------------------------------------------------------
