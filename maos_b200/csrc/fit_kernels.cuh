@@ -2,59 +2,96 @@
 //
 // The reference's default GPU fit (cuda/solve.cu cusolve_sparse, cumuv_t)
 // applies FR and FL as cuSPARSE csrmv plus two cuBLAS gemv per operator,
-// one instance at a time.  Here every operator is two launches for all
-// instances sharing the matrices:
+// one instance at a time.  Here:
 //   k_lr_dot   t[b][q] = V_q' x_b (FP64 block partials, the last block to
 //              arrive adds them in a fixed order)
 //   k_spmv_lr  y_b = M x_b - U t_b, M in CSR as (column, value) pairs read
 //              once per group of NI instances, optionally + p.Ap partials and
 //              alpha for CG.
-// Every instance's sums are formed independently of the others (a warp per
-// row, each lane holding NI instance sums, a butterfly over the warp), so
-// results do not depend on which instances run together.
+// Inside the CG, k_cg_step (tomo_kernels.cuh) leaves t = V' p with the new p,
+// so an iteration is two launches.  Every instance's sums are formed
+// independently of the others (a warp per row, each lane holding NI instance
+// sums, reduced over the warp), so results do not depend on which instances
+// run together.
 #pragma once
 #include "tomo_kernels.cuh"
 
 namespace mb {
 
-constexpr int kMaxLr = 16;  // low-rank columns (FR: fit directions; FL: + NW)
-
-// grid: (ceil(n/256), nb); part [nb][nq][gridDim.x]; t [nb][kMaxLr]
+// NI instances share a thread's E elements of every column of V.
+// grid: (ceil(n / (kThreads * E)), ceil(nb / NI)); part [nb][nq][gridDim.x]; t [nb][kMaxLr]
+template <int NI, int E>
 __global__ void __launch_bounds__(kThreads)
 k_lr_dot(const float *__restrict__ x, const float *__restrict__ V, int nq, long n, double *__restrict__ part,
-         float *__restrict__ t, unsigned *__restrict__ cnt, const int *__restrict__ act) {
+         float *__restrict__ t, unsigned *__restrict__ cnt, int nb, const int *__restrict__ act) {
     pdl_enter();
-    if (inactive(act, blockIdx.y)) return;
-    __shared__ double sh[kThreads / 32][kMaxLr];
-    const int b = blockIdx.y;
+    const int b0 = blockIdx.y * NI;
+    bool on[NI];
+    bool any = false;
+#pragma unroll
+    for (int u = 0; u < NI; u++) {
+        on[u] = b0 + u < nb && !inactive(act, b0 + u);
+        any |= on[u];
+    }
+    if (!any) return;
+    __shared__ double sh[kThreads / 32][kMaxLr][NI];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const long j = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    const float xv = (j < n) ? x[(size_t)b * n + j] : 0.f;
+    const long j0 = (long)blockIdx.x * (kThreads * E) + threadIdx.x;
+    float xv[NI][E];
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+        const long j = j0 + e * kThreads;
+#pragma unroll
+        for (int u = 0; u < NI; u++) xv[u][e] = on[u] && j < n ? x[(size_t)(b0 + u) * n + j] : 0.f;
+    }
+#pragma unroll 2
     for (int q = 0; q < nq; q++) {
-        double v = (j < n) ? (double)V[(size_t)q * n + j] * (double)xv : 0.0;
-        v = warp_sum(v);
-        if (lane == 0) sh[wid][q] = v;
+        float vv[E];
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            const long j = j0 + e * kThreads;
+            vv[e] = j < n ? V[(size_t)q * n + j] : 0.f;
+        }
+        double v[NI];
+#pragma unroll
+        for (int u = 0; u < NI; u++) {
+            v[u] = 0;
+#pragma unroll
+            for (int e = 0; e < E; e++) v[u] += (double)vv[e] * (double)xv[u][e];
+        }
+        const int at = warp_sum_many<NI>(v);
+        if (lane % (32 / NI) == 0) sh[wid][q][at] = v[0];
     }
     __syncthreads();
-    if (threadIdx.x < nq) {
+    for (int e = threadIdx.x; e < nq * NI; e += kThreads) {
+        const int q = e / NI, u = e - q * NI;
         double s = 0;
 #pragma unroll
-        for (int w = 0; w < kThreads / 32; w++) s += sh[w][threadIdx.x];
-        part[((size_t)b * nq + threadIdx.x) * gridDim.x + blockIdx.x] = s;
+        for (int w = 0; w < kThreads / 32; w++) s += sh[w][q][u];
+        if (b0 + u < nb) part[((size_t)(b0 + u) * nq + q) * gridDim.x + blockIdx.x] = s;
     }
-    if (last_block(cnt + b, gridDim.x)) {
-        for (int q = wid; q < nq; q += kThreads / 32) {
-            const double s = warp_sum_fresh(part + ((size_t)b * nq + q) * gridDim.x, gridDim.x);
-            if (lane == 0) t[(size_t)b * kMaxLr + q] = (float)s;
+    if (last_block(cnt + b0, gridDim.x)) {
+        for (int e = wid; e < nq * NI; e += kThreads / 32) {
+            const int q = e / NI, u = e - q * NI;
+            if (b0 + u >= nb || inactive(act, b0 + u)) continue;
+            const double s = warp_sum_fresh(part + ((size_t)(b0 + u) * nq + q) * gridDim.x, gridDim.x);
+            if (lane == 0) t[(size_t)(b0 + u) * kMaxLr + q] = (float)s;
         }
-        if (threadIdx.x == 0) cnt[b] = 0;
+        if (threadIdx.x == 0) cnt[b0] = 0;
     }
 }
 
 // y[b][i] = sum_e M[i][e] x[b][col_e] - sum_q U[q*nrow + i] t[b][q] (+ add[b][i]).
-// One warp per row (8 rows per CTA); grid: (ceil(nb/NI), ceil(nrow/8)).
+// One warp takes kSpmvRows rows one after the other (the CTA's barriers, its
+// p.Ap partial and its arrival are shared by them; four entries per lane are
+// in flight); the NI sums are reduced over the warp by exchanging halves, so a
+// row costs NI + 1 shuffles instead of 5 NI.
+// grid: (ceil(nb/NI), ceil(nrow / kSpmvBlock)).
 // With dot_part: the p.Ap partials (dot_x = p) per CTA, [nb][gridDim.y], and
 // the last CTA of each instance group leaves alpha_k = (r.z)_k / p.Ap.
+constexpr int kSpmvRows = 2;
+constexpr int kSpmvBlock = kThreads / 32 * kSpmvRows;  // rows per CTA
+
 template <int NI>
 __global__ void __launch_bounds__(kThreads)
 k_spmv_lr(const int *__restrict__ rp, const GatherW *__restrict__ ent, int nrow, long ncol,
@@ -73,45 +110,57 @@ k_spmv_lr(const int *__restrict__ rp, const GatherW *__restrict__ ent, int nrow,
     }
     if (!any) return;  // uniform over the instance group
     __shared__ double sh[kThreads / 32][NI];
+    __shared__ float s_t[NI][kMaxLr];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int row = blockIdx.y * (kThreads / 32) + wid;
-    float acc[NI];
-#pragma unroll
-    for (int q = 0; q < NI; q++) acc[q] = 0.f;
-    if (row < nrow) {
-        const int e1 = rp[row + 1];
-        for (int e = rp[row] + lane; e < e1; e += 32) {
-            const GatherW g = ent[e];
-#pragma unroll
-            for (int q = 0; q < NI; q++)
-                if (on[q]) acc[q] += g.w * x[(size_t)(b0 + q) * ncol + g.i];
+    const int row0 = blockIdx.y * kSpmvBlock + wid;
+    if (nq) {
+        if (threadIdx.x < NI * kMaxLr) {
+            const int u = threadIdx.x / kMaxLr;
+            s_t[u][threadIdx.x % kMaxLr] = u < ni ? t[(size_t)(b0 + u) * kMaxLr + threadIdx.x % kMaxLr] : 0.f;
         }
+        __syncthreads();
     }
-#pragma unroll
-    for (int q = 0; q < NI; q++)
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
-    // lane q finishes instance b0 + q
-    float mine = 0.f;
-    bool mon = false;
-#pragma unroll
-    for (int q = 0; q < NI; q++)
-        if (lane == q) {
-            mine = acc[q];
-            mon = on[q];
-        }
+    const float *xb = x + (size_t)b0 * ncol;
     double dv = 0.0;
-    if (row < nrow && lane < NI && mon) {
-        const int b = b0 + lane;
+    int inst = 0;  // the instance whose sum this lane holds after the reduction
+    bool out = false;
+#pragma unroll
+    for (int rr = 0; rr < kSpmvRows; rr++) {
+        const int row = row0 + rr * (kThreads / 32);
+        if (row >= nrow) break;
+        const float uv = lane < nq ? U[(size_t)lane * nrow + row] : 0.f;
+        float acc[NI];
+#pragma unroll
+        for (int q = 0; q < NI; q++) acc[q] = 0.f;
+        const int e1 = rp[row + 1];
+        for (int e = rp[row] + lane; e < e1; e += 4 * 32) {
+            GatherW g[4];
+#pragma unroll
+            for (int c = 0; c < 4; c++) g[c] = e + 32 * c < e1 ? ent[e + 32 * c] : GatherW{0, 0.f};
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                if (e + 32 * c >= e1) break;
+#pragma unroll
+                for (int q = 0; q < NI; q++)
+                    if (on[q]) acc[q] += g[c].w * xb[(size_t)q * ncol + g[c].i];
+            }
+        }
+        inst = warp_sum_many<NI>(acc);
+        out = lane % (32 / NI) == 0 && inst < ni && !inactive(act, b0 + inst);
         float lr = 0.f;
-        for (int q = 0; q < nq; q++) lr += U[(size_t)q * nrow + row] * t[(size_t)b * kMaxLr + q];
-        float v = mine - lr;
-        if (add) v += add[(size_t)b * nrow + row];
-        y[(size_t)b * nrow + row] = v;
-        if (dot_part) dv = (double)v * (double)dot_x[(size_t)b * nrow + row];
+        for (int q = 0; q < nq; q++) lr += __shfl_sync(0xffffffffu, uv, q) * s_t[inst][q];
+        if (out) {
+            const size_t o = (size_t)(b0 + inst) * nrow + row;
+            float v = acc[0] - lr;
+            if (add) v += add[o];
+            y[o] = v;
+            if (dot_part) dv += (double)v * (double)dot_x[o];
+        }
     }
     if (!dot_part) return;  // uniform
-    if (lane < NI) sh[wid][lane] = dv;
+    if (threadIdx.x < NI * (kThreads / 32)) sh[threadIdx.x / NI][threadIdx.x % NI] = 0.0;
+    __syncthreads();
+    if (out) sh[wid][inst] = dv;
     __syncthreads();
     if (threadIdx.x < ni) {  // instances past nbatch have no row in dot_part
         double s = 0;

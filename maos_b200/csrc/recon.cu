@@ -176,6 +176,11 @@ struct Recon {
 
     DevBuf<cplx> spec, spec2;               // half spectra
 
+    struct CgBufs {
+        float *x, *r, *p, *z, *Ap, *rhs;
+        double *pap, *rr, *rz, *bb;
+        CgScal S;
+    };
     // state and work buffers
     DevBuf<float> x, r, p, z, Ap, rhs, opd, grad, gin;
     DevBuf<double> tt_part, pap_part, rr_part, rz_part, bb_part, sc;
@@ -219,7 +224,7 @@ struct Recon {
     DevBuf<float> fslv;
     // assembled fit (fit_sparse): FR, FL as CSR (column, value) plus low rank
     bool fit_sparse = false;
-    int nfr = 0, nfl = 0, nrb_a = 0;       // low-rank columns; 8-row blocks over the actuators
+    int nfr = 0, nfl = 0, nrb_a = 0;       // low-rank columns; CTAs of k_spmv_lr over the actuators
     DevBuf<int> frm_rp, flm_rp;
     DevBuf<GatherW> frm_e, flm_e;
     DevBuf<float> fru, frv, flu, flv;
@@ -229,6 +234,8 @@ struct Recon {
     void spmv(const DevBuf<int> &rp, const DevBuf<GatherW> &e, int nrow, long ncol, const float *xin, float *out,
               const float *U, int nq, const float *add, double *dot, int k, cudaStream_t s);
     void lr_dot(const float *xin, const float *V, int nq, long n, cudaStream_t s);
+    static bool cg_step_fits(long n) { return n <= 8L * 8 * kStepThreads; }
+    bool cg_step(const CgBufs &B, long n, int k, int iters, int init, const float *V, int nq, cudaStream_t s);
     void build_fit_sparse(const mb_fit_sparse_desc *f);
     void alloc_fit_state();
 
@@ -322,17 +329,13 @@ struct Recon {
     void form_fdpcg_data(const double *neam);
     void set_fdpcg_mode(int mode);
     void enqueue_solve(cudaStream_t s);
-    struct CgBufs {
-        float *x, *r, *p, *z, *Ap, *rhs;
-        double *pap, *rr, *rz, *bb;
-        CgScal S;
-    };
     using AmulFn = std::function<void(const float *, float *, double *, int)>;
     // preconditioners return true when they also left p = z + beta p
     using MmulFn = std::function<bool(float *, float *, double *, int, int)>;
     using XrMmulFn = std::function<bool(int)>;
     void enqueue_cg(const CgBufs &B, long n, int nblk, int iters, const AmulFn &Amul,
-                    const MmulFn &Mmul, cudaStream_t s, const XrMmulFn &XrMmul = XrMmulFn());
+                    const MmulFn &Mmul, cudaStream_t s, const XrMmulFn &XrMmul = XrMmulFn(),
+                    const float *V = nullptr, int nq = 0);
     // One CG solve taken apart at its operator applications, so that a
     // ReconGroup can apply the operator of several reconstructors in one
     // launch: after A x -> cg_init; after A p_k -> cg_post (true: done).
@@ -343,13 +346,16 @@ struct Recon {
         MmulFn Mmul;
         XrMmulFn XrMmul;
         float *zp;
+        const float *V = nullptr;  // low-rank columns whose t = V' p cg_step leaves for the next A p
+        int nq = 0;
     };
     void cg_init(CgRun &c, int k, cudaStream_t s);
     bool cg_post(CgRun &c, int k, cudaStream_t s);
     CgRun solve_run(cudaStream_t s);  // the tomography CG (its preconditioner launched on s)
     void op_rhs_gp(const float *g, cudaStream_t s);  // the first launch of op_rhs (gradient weighting)
     void op_fitR(const float *xin, float *out, cudaStream_t s);
-    void op_fitL(const float *ain, float *out, double *dot_part, cudaStream_t s, int k = 0);
+    // t_ready: V' ain is already in lr_t (left by cg_step)
+    void op_fitL(const float *ain, float *out, double *dot_part, cudaStream_t s, int k = 0, bool t_ready = false);
     void enqueue_fit(cudaStream_t s);
     void time_stages(int reps, float *ms, double *bytes, int *launches);
     void capture_graph();
@@ -1473,6 +1479,7 @@ bool Recon::op_fdpcg(float *rin, float *zout, double *rzp, cudaStream_t s, int k
 void Recon::cg_init(CgRun &c, int k, cudaStream_t s) {
     // after Ap = A x: r = b - A x, b.b, z = M r, (r.z)_k, p = z
     const CgBufs &B = c.B;
+    if (!c.Mmul && cg_step(B, c.n, k, c.iters, 1, c.V, c.nq, s)) return;
     launch(k_cg_init_r, dim3(c.nblk, nb), dim3(kThreads), 0, s, B.rhs, B.Ap, B.r, B.bb, c.n, B.S, c.iters, act());
     bool pdone = false;
     if (c.Mmul) {
@@ -1488,6 +1495,7 @@ void Recon::cg_init(CgRun &c, int k, cudaStream_t s) {
 bool Recon::cg_post(CgRun &c, int k, cudaStream_t s) {
     // after Ap = A p_k (whose last block left alpha_k)
     const CgBufs &B = c.B;
+    if (!c.Mmul && cg_step(B, c.n, k, c.iters, 0, c.V, c.nq, s)) return k + 1 == c.iters;
     bool pdone;
     if (c.XrMmul && k + 1 < c.iters) {
         pdone = c.XrMmul(k);  // x, r update and preconditioner; beta_k (and p, when it says so)
@@ -1503,6 +1511,19 @@ bool Recon::cg_post(CgRun &c, int k, cudaStream_t s) {
     return false;
 }
 
+// The vector part of an unpreconditioned iteration as one cluster launch;
+// false where an instance's vector does not fit a cluster's registers (8
+// elements per thread of 8 CTAs; then the separate kernels run).  As few CTAs
+// as keep 4 elements per thread.
+bool Recon::cg_step(const CgBufs &B, long n, int k, int iters, int init, const float *V, int nq, cudaStream_t s) {
+    if (!cg_step_fits(n)) return false;
+    const int C = (int)std::min(8L, (n + 4L * kStepThreads - 1) / (4L * kStepThreads));
+    const auto kern = n <= 4L * kStepThreads * C ? k_cg_step<4> : k_cg_step<8>;
+    launch_cluster(kern, dim3(C, nb), dim3(kStepThreads), 0, s, C, B.x, B.r, B.p, (const float *)B.Ap,
+                   (const float *)B.rhs, n, B.S, k, iters, init, V, nq, lr_t.p, act());
+    return true;
+}
+
 // (Preconditioned) CG with FP64 scalars, the schedule of lib/pcg.c:28: the
 // residual is recomputed from x every kCgRestart = 100 iterations as the
 // reference's CPU solver does (its GPU solver, cuda/pcg.cu:87, every 500),
@@ -1511,8 +1532,8 @@ bool Recon::cg_post(CgRun &c, int k, cudaStream_t s) {
 // XrMmul, when given, performs the x/r update of a non-final iteration
 // together with the preconditioner.
 void Recon::enqueue_cg(const CgBufs &B, long n, int nblk, int iters, const AmulFn &Amul,
-                       const MmulFn &Mmul, cudaStream_t s, const XrMmulFn &XrMmul) {
-    CgRun c{B, n, nblk, iters, Mmul, XrMmul, Mmul ? B.z : B.r};
+                       const MmulFn &Mmul, cudaStream_t s, const XrMmulFn &XrMmul, const float *V, int nq) {
+    CgRun c{B, n, nblk, iters, Mmul, XrMmul, Mmul ? B.z : B.r, V, nq};
     Amul(B.x, B.Ap, nullptr, 0);
     cg_init(c, 0, s);
     for (int k = 0; k < iters; k++) {
@@ -1551,7 +1572,7 @@ void Recon::enqueue_solve(cudaStream_t s) {
 // y = M x - U (V'x) for all instances: one warp per row, NI instances per CTA.
 void Recon::spmv(const DevBuf<int> &rp, const DevBuf<GatherW> &e, int nrow, long ncol, const float *xin, float *out,
                  const float *U, int nq, const float *add, double *dot, int k, cudaStream_t s) {
-    const unsigned ry = (unsigned)((nrow + kThreads / 32 - 1) / (kThreads / 32));
+    const unsigned ry = (unsigned)((nrow + kSpmvBlock - 1) / kSpmvBlock);
     const CgScal S = dot ? fscal() : CgScal{};
     const float *dx = dot ? xin : nullptr;
 #define MB_SPMV(NI)                                                                                            \
@@ -1566,7 +1587,15 @@ void Recon::spmv(const DevBuf<int> &rp, const DevBuf<GatherW> &e, int nrow, long
 
 // t[b][q] = V_q' x_b (FP64 partials, fixed-order total)
 void Recon::lr_dot(const float *xin, const float *V, int nq, long n, cudaStream_t s) {
-    launch(k_lr_dot, dim3(nblocks(n), nb), dim3(kThreads), 0, s, xin, V, nq, n, lr_part.p, lr_t.p, lr_cnt.p, act());
+    // 4 instances and 4 elements per thread read V a quarter as often and reduce
+    // once for 16 products, but leave few CTAs: 30 m layers (9 x 27,648), 256
+    // instances 56 -> 38 us, 6 instances 6.5 -> 13 us
+    if (nb >= 64)
+        launch(k_lr_dot<4, 4>, dim3(nblocks(n, 4 * kThreads), (nb + 3) / 4), dim3(kThreads), 0, s, xin, V, nq, n,
+               lr_part.p, lr_t.p, lr_cnt.p, nb, act());
+    else
+        launch(k_lr_dot<1, 1>, dim3(nblocks(n), nb), dim3(kThreads), 0, s, xin, V, nq, n, lr_part.p, lr_t.p, lr_cnt.p,
+               nb, act());
 }
 
 // FitR: sum_f wt_f HA_f^T (W0 - W1 W1^T) Hxp_f x   (recon_utils.c:483, fit.cu:190)
@@ -1588,9 +1617,9 @@ void Recon::op_fitR(const float *xin, float *out, cudaStream_t s) {
 // FitL: sum_f wt_f HA_f^T (W0 - W1 W1^T) HA_f a + NW NW^T a + actslave a
 //       (recon_utils.c:536, fit.cu:213-235)
 // assembled: FL.M a - FL.U (FL.V' a)                 (lib/muv.c:37, solve.cu:36)
-void Recon::op_fitL(const float *ain, float *out, double *dot_part, cudaStream_t s, int k) {
+void Recon::op_fitL(const float *ain, float *out, double *dot_part, cudaStream_t s, int k, bool t_ready) {
     if (fit_sparse) {
-        if (nfl) lr_dot(ain, flv.p, nfl, nact, s);
+        if (nfl && !t_ready) lr_dot(ain, flv.p, nfl, nact, s);
         spmv(flm_rp, flm_e, (int)nact, nact, ain, out, nfl ? flu.p : nullptr, nfl, nullptr, dot_part, k, s);
         return;
     }
@@ -1614,8 +1643,9 @@ void Recon::op_fitL(const float *ain, float *out, double *dot_part, cudaStream_t
 void Recon::enqueue_fit(cudaStream_t s) {
     op_fitR(x.p, frhs.p, s);
     CgBufs B{fa.p, fr.p, fp.p, fr.p, fAp.p, frhs.p, f_pap.p, f_rr.p, f_rz.p, f_bb.p, fscal()};
-    AmulFn A = [&](const float *in, float *out, double *dot, int k) { op_fitL(in, out, dot, s, k); };
-    enqueue_cg(B, nact, nblk_a, fit_maxit, A, MmulFn(), s);
+    const bool lr = fit_sparse && nfl && cg_step_fits(nact);
+    AmulFn A = [&](const float *in, float *out, double *dot, int k) { op_fitL(in, out, dot, s, k, lr && in == fp.p); };
+    enqueue_cg(B, nact, nblk_a, fit_maxit, A, MmulFn(), s, XrMmulFn(), lr ? flv.p : nullptr, lr ? nfl : 0);
 }
 
 // CSC (the reference's dsp) -> CSR rows of (column, value) pairs.
@@ -1646,12 +1676,12 @@ static void upload_f32(DevBuf<float> &d, const double *h, size_t n) {
 // CG state and scratch of the fit (both forms), sized by nact.
 void Recon::alloc_fit_state() {
     nblk_a = (int)nblocks(nact);
-    nrb_a = (int)((nact + kThreads / 32 - 1) / (kThreads / 32));
+    nrb_a = (int)((nact + kSpmvBlock - 1) / kSpmvBlock);
     MB_REQUIRE(nrb_a < 65535, "fit: too many actuators (%ld)", nact);
     fnsc = fit_maxit + 3;
     const size_t NA = (size_t)nb * nact;
     fa.alloc(NA); fr.alloc(NA); fp.alloc(NA); fAp.alloc(NA); frhs.alloc(NA);
-    // the p.Ap partials of the sparse operator are per 8-row block, of the grid one per 256 actuators
+    // the p.Ap partials of the sparse operator are per k_spmv_lr CTA, of the grid one per 256 actuators
     f_pap.alloc((size_t)nb * std::max(nblk_a, nrb_a)); f_rr.alloc((size_t)nb * nblk_a);
     f_rz.alloc((size_t)nb * nblk_a); f_bb.alloc((size_t)nb * nblk_a);
     fsc.alloc((size_t)nb * fnsc);

@@ -71,6 +71,32 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
+// Sums over the warp of N values per lane (N a power of two up to 32), by
+// exchanging halves: each step, a lane keeps half of its values and adds the
+// partner's.  v[0] is then the sum of value `return` (the same in each of the
+// 32 / N consecutive lanes that hold it).  The sums are those of a butterfly
+// from 16 down to 1.
+template <int N, class T>
+__device__ __forceinline__ int warp_sum_many(T (&v)[N]) {
+    const int lane = threadIdx.x & 31;
+    int at = 0, o = 16;
+#pragma unroll
+    for (int n = N / 2; n >= 1; n /= 2, o /= 2) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < n; i++) {
+            const T give = up ? v[i] : v[i + n], keep = up ? v[i + n] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+        at += up ? n : 0;
+    }
+#pragma unroll
+    for (; o >= 1; o /= 2) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    return at;
+}
+
+constexpr int kMaxLr = 16;  // low-rank columns of the assembled fit (FR: fit directions; FL: + NW)
+
 // Block-wide sum of one double; result valid in thread 0.
 __device__ __forceinline__ double block_sum(double v, double *sh) {
     v = warp_sum(v);
@@ -1699,6 +1725,148 @@ k_fd_data(FdGeomDev G, const int4 *__restrict__ mem, const int2 *__restrict__ bl
 
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ double dsm_peer_f64(const double *local, unsigned rank) {
+    unsigned ra;
+    double v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                 : "=r"(ra) : "r"((unsigned)__cvta_generic_to_shared(local)), "r"(rank));
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(ra) : "memory");
+    return v;
+}
+
+// The vector part of an unpreconditioned CG iteration in one launch, a
+// thread-block cluster per instance: x += alpha p, r -= alpha Ap, r.r over the
+// cluster, beta, p = r + beta p, and (fit) t = V' p, what the next A p needs
+// of the low-rank term.  init: r = b - Ap (Ap = A x), b.b, r.r, p = r, t.  The
+// elements stay in registers between the passes.  The last iteration leaves
+// the residual instead of p.  Launch-bound: one launch of 4-9 us where the
+// update of x and r, the update of p and V' p took three of 3.7, 1.8 and 4-14
+// us (8 m LTAO tomography and 30 m fit, 1 to 32 instances).
+// grid: (cluster size, nb), block: kStepThreads, E elements per thread.
+constexpr int kStepThreads = 512;
+
+template <int E>
+__global__ void __launch_bounds__(kStepThreads)
+k_cg_step(float *__restrict__ x, float *__restrict__ r, float *__restrict__ p, const float *__restrict__ Ap,
+          const float *__restrict__ bvec, long n, CgScal S, int k, int iters, int init, const float *__restrict__ V,
+          int nq, float *__restrict__ t, const int *__restrict__ act) {
+    pdl_enter();
+    if (inactive(act, blockIdx.y)) return;  // the whole cluster
+    __shared__ double sh[kStepThreads / 32], sh2[kStepThreads / 32], s_part[2], s_lr[kMaxLr];
+    __shared__ double s_w[kStepThreads / 32][kMaxLr];
+    __shared__ float s_beta;
+    const int b = blockIdx.y, C = gridDim.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const size_t ob = (size_t)b * n;
+    const long j0 = (long)blockIdx.x * (kStepThreads * E) + threadIdx.x;
+    float rv[E], pv[E];
+    double rr = 0, bb = 0;
+    if (init) {
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            const long j = j0 + e * kStepThreads;
+            const float bv = j < n ? bvec[ob + j] : 0.f;
+            rv[e] = j < n ? bv - Ap[ob + j] : 0.f;
+            pv[e] = 0.f;
+            bb += (double)bv * bv;
+            rr += (double)rv[e] * rv[e];
+        }
+    } else {
+        const float a = S.ab[2 * b];
+        float xv[E], av[E];
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            const long j = j0 + e * kStepThreads;
+            pv[e] = j < n ? p[ob + j] : 0.f;
+            rv[e] = j < n ? r[ob + j] : 0.f;
+            xv[e] = j < n ? x[ob + j] : 0.f;
+            av[e] = j < n ? Ap[ob + j] : 0.f;
+        }
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            const long j = j0 + e * kStepThreads;
+            xv[e] += a * pv[e];
+            rv[e] -= a * av[e];
+            if (j < n) x[ob + j] = xv[e];
+            rr += (double)rv[e] * rv[e];
+        }
+    }
+    // r.r (and b.b) over the cluster: every rank adds the partials in rank order
+    rr = block_sum(rr, sh);
+    if (init) bb = block_sum(bb, sh2);
+    if (threadIdx.x == 0) {
+        s_part[0] = rr;
+        s_part[1] = bb;
+    }
+    if (C > 1) cluster_sync_all();
+    if (threadIdx.x == 0) {
+        for (int c = 0; c < C; c++) {
+            if (c == 0) rr = bb = 0;
+            rr += C > 1 ? dsm_peer_f64(&s_part[0], c) : s_part[0];
+            if (init) bb += C > 1 ? dsm_peer_f64(&s_part[1], c) : s_part[1];
+        }
+        double *sc = S.sc + (size_t)b * S.nsc;
+        double be = 0;
+        if (init) {  // start (or restart, lib/pcg.c:61) at iteration k
+            if (blockIdx.x == 0) {
+                sc[iters + 1] = bb;
+                sc[k] = rr;
+            }
+        } else if (k + 1 == iters) {
+            if (blockIdx.x == 0) {
+                const double res = sqrt(rr / sc[iters + 1]);
+                sc[iters + 2] = res;
+                S.res[b] = (float)res;
+            }
+        } else {
+            be = rr / sc[k];
+            if (!isfinite(be)) be = 0;
+            if (blockIdx.x == 0) sc[k + 1] = rr;
+        }
+        s_beta = (float)be;
+    }
+    __syncthreads();
+    const bool last = !init && k + 1 == iters;
+    const float be = s_beta;
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+        const long j = j0 + e * kStepThreads;
+        pv[e] = init ? rv[e] : rv[e] + be * pv[e];
+        if (j < n) {
+            r[ob + j] = rv[e];
+            if (!last) p[ob + j] = pv[e];
+        }
+    }
+    if (nq && !last) {
+        for (int q0 = 0; q0 < nq; q0 += 4) {
+            double v[4] = {0, 0, 0, 0};
+#pragma unroll
+            for (int e = 0; e < E; e++) {
+                const long j = j0 + e * kStepThreads;
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if (q0 + u < nq && j < n) v[u] += (double)V[(size_t)(q0 + u) * n + j] * (double)pv[e];
+            }
+            const int at = warp_sum_many<4>(v);
+            if (lane % 8 == 0) s_w[wid][q0 + at] = v[0];
+        }
+        __syncthreads();
+        if (threadIdx.x < nq) {
+            double v = 0;
+#pragma unroll
+            for (int w = 0; w < kStepThreads / 32; w++) v += s_w[w][threadIdx.x];
+            s_lr[threadIdx.x] = v;
+        }
+        if (C > 1) cluster_sync_all();
+        else __syncthreads();
+        if (blockIdx.x == 0 && threadIdx.x < nq) {
+            double v = 0;
+            for (int c = 0; c < C; c++) v += C > 1 ? dsm_peer_f64(&s_lr[threadIdx.x], c) : s_lr[threadIdx.x];
+            t[(size_t)b * kMaxLr + threadIdx.x] = (float)v;
+        }
+    }
+    if (C > 1) cluster_sync_all();  // peers are done reading this CTA's partials
 }
 
 // Inverse: half spectra H -> z (instance-major), plus the r.z partial of this
