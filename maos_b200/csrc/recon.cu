@@ -611,7 +611,7 @@ int Recon::hxt_window(int l, int rows) const {
             if (hi > 0) ky = std::max(ky, hi - lo);
         }
     }
-    const int c = hxt_chunk(hxt_width(kx));
+    const int c = hxt_chunk(hxt_width(kx), rows);
     return (ky + c - 1) / c * c;
 }
 

@@ -661,7 +661,7 @@ constexpr int kHxtThreads = 128;
 // Tables of the transpose (device), all of one layer at the layer's own width.
 struct HxtLayer {
     int k;             // width of the column lists: 2, 3, 4, 6 or 8
-    int n;             // pupil rows of a row window (a multiple of hxt_chunk(k))
+    int n;             // pupil rows of a row window (a multiple of hxt_chunk(k, RT))
     int xoff, roff;    // first column list, first row window (of WFS 0) of the layer
     int woff, groups;  // first weight vector; row groups of RT rows
     int blocks;        // CTAs of the layer
@@ -675,7 +675,12 @@ struct HxtIndex {
     const int *y0;     // [roff + w*groups + g]: first pupil row, -1: none
     const float *yw;   // [(woff + (w*groups + g)*n + i) * RT + r]: weight of pupil row y0 + i to layer row g*RT + r
 };
-__host__ __device__ constexpr int hxt_chunk(int k) { return k <= 4 ? 5 : 2; }  // pupil rows whose loads go together
+// Pupil rows whose loads go together: what RT rows of a layer sampled as the
+// pupil need (a layer at half the sampling takes two chunks).
+__host__ __device__ constexpr int hxt_chunk(int k, int rt) { return k > 4 ? 2 : rt == 4 ? 5 : rt == 2 ? 3 : 2; }
+// WFS whose loads go together: with one row per thread the launch is too small
+// to hide a WFS's two round trips behind other warps.
+__host__ __device__ constexpr int hxt_wfs(int k, int rt) { return rt == 1 && k <= 4 ? 3 : 1; }
 
 // Arguments of one k_hxt_rows launch.
 struct HxtArgs {
@@ -711,40 +716,62 @@ __device__ __forceinline__ void load_row_weights(float (&w)[RT], const float *p)
 template <int K, int RT>
 __device__ __forceinline__ void hxt_column(const HxtArgs &A, const HxtLayer &H, int nx, int b, int g, int jx,
                                            float (&acc)[RT]) {
-    constexpr int C = hxt_chunk(K);
+    constexpr int C = hxt_chunk(K, RT), NW = hxt_wfs(K, RT);
     const int stride = A.ostride;
-    for (int w = 0; w < A.nwfs; w++) {
-        const int x0 = A.ix.x0[H.xoff + w * nx + jx];
-        const int rw = w * H.groups + g, y0 = A.ix.y0[H.roff + rw];
-        if (x0 < 0 || y0 < 0) continue;  // outside this WFS's footprint
-        float xw[K];
-        const float *xp = A.ix.xw + (size_t)(H.xoff + w * nx) * kMaxPad + jx;
+    for (int w0 = 0; w0 < A.nwfs; w0 += NW) {
+        int x0[NW], y0[NW];
+        bool in[NW];
 #pragma unroll
-        for (int e = 0; e < K; e++) xw[e] = xp[e * nx];
-        const float *o = A.o + ((size_t)(b * A.nwfs + w) * A.orows + y0) * stride + x0;
-        const float *yw = A.ix.yw + ((size_t)H.woff + (size_t)rw * H.n) * RT;
-        float s[RT];
+        for (int u = 0; u < NW; u++) {
+            const int w = min(w0 + u, A.nwfs - 1);
+            x0[u] = A.ix.x0[H.xoff + w * nx + jx];
+            y0[u] = A.ix.y0[H.roff + w * H.groups + g];
+        }
 #pragma unroll
-        for (int r = 0; r < RT; r++) s[r] = 0.f;
-        for (int i = 0; i < H.n; i += C, o += C * stride, yw += C * RT) {
-            float v[C][K], wy[C][RT];
+        for (int u = 0; u < NW; u++) in[u] = w0 + u < A.nwfs && x0[u] >= 0 && y0[u] >= 0;  // in the WFS's footprint
+        if (NW == 1 && !in[0]) continue;
+        float xw[NW][K], s[NW][RT];
+        const float *o[NW], *yw[NW];
 #pragma unroll
-            for (int q = 0; q < C; q++) {
+        for (int u = 0; u < NW; u++) {
+            const int w = min(w0 + u, A.nwfs - 1);
+            const float *xp = A.ix.xw + (size_t)(H.xoff + w * nx) * kMaxPad + jx;
 #pragma unroll
-                for (int e = 0; e < K; e++) v[q][e] = o[q * stride + e];
-                load_row_weights<RT>(wy[q], yw + q * RT);
-            }
+            for (int e = 0; e < K; e++) xw[u][e] = xp[e * nx];
+            o[u] = A.o + ((size_t)(b * A.nwfs + w) * A.orows + max(y0[u], 0)) * stride + max(x0[u], 0);
+            yw[u] = A.ix.yw + ((size_t)H.woff + (size_t)(w * H.groups + g) * H.n) * RT;
 #pragma unroll
-            for (int q = 0; q < C; q++) {
-                float t = 0.f;
+            for (int r = 0; r < RT; r++) s[u][r] = 0.f;
+        }
+        for (int i = 0; i < H.n; i += C) {
+            float v[NW][C][K], wy[NW][C][RT];
 #pragma unroll
-                for (int e = 0; e < K; e++) t += xw[e] * v[q][e];
+            for (int u = 0; u < NW; u++)
 #pragma unroll
-                for (int r = 0; r < RT; r++) s[r] += wy[q][r] * t;
+                for (int q = 0; q < C; q++) {
+#pragma unroll
+                    for (int e = 0; e < K; e++) v[u][q][e] = o[u][q * stride + e];
+                    load_row_weights<RT>(wy[u][q], yw[u] + q * RT);
+                }
+#pragma unroll
+            for (int u = 0; u < NW; u++) {
+#pragma unroll
+                for (int q = 0; q < C; q++) {
+                    float t = 0.f;
+#pragma unroll
+                    for (int e = 0; e < K; e++) t += xw[u][e] * v[u][q][e];
+#pragma unroll
+                    for (int r = 0; r < RT; r++) s[u][r] += wy[u][q][r] * t;
+                }
+                o[u] += C * stride;
+                yw[u] += C * RT;
             }
         }
 #pragma unroll
-        for (int r = 0; r < RT; r++) acc[r] += s[r];
+        for (int u = 0; u < NW; u++)
+            if (in[u])
+#pragma unroll
+                for (int r = 0; r < RT; r++) acc[r] += s[u][r];
     }
 }
 
