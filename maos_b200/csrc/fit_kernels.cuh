@@ -6,8 +6,8 @@
 //   k_lr_dot   t[b][q] = V_q' x_b (FP64 block partials, the last block to
 //              arrive adds them in a fixed order)
 //   k_spmv_lr  y_b = M x_b - U t_b, M in CSR as (column, value) pairs read
-//              once per group of NI instances, optionally + p.Ap partials and
-//              alpha for CG.
+//              once per group of NI instances, optionally + p.Ap partials for
+//              the CG.
 // Inside the CG, k_cg_step (tomo_kernels.cuh) leaves t = V' p with the new p,
 // so an iteration is two launches.  Every instance's sums are formed
 // independently of the others (a warp per row, each lane holding NI instance
@@ -81,23 +81,70 @@ k_lr_dot(const float *__restrict__ x, const float *__restrict__ V, int nq, long 
     }
 }
 
+// The NI instances of a group with their values of one index side by side:
+// out[(group*n + j)*NI + q] = x[(group*NI + q)*n + j], 0 past the last
+// instance.  grid: (ceil(n / kThreads), groups).
+template <int NI>
+__global__ void __launch_bounds__(kThreads)
+k_interleave(const float *__restrict__ x, float *__restrict__ out, long n, int nb) {
+    pdl_enter();
+    const long j = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= n) return;
+    const int b0 = blockIdx.y * NI;
+    float v[NI];
+#pragma unroll
+    for (int q = 0; q < NI; q++) v[q] = b0 + q < nb ? x[(size_t)(b0 + q) * n + j] : 0.f;
+    float *o = out + ((size_t)blockIdx.y * n + j) * NI;
+    if constexpr (NI % 4 == 0) {
+#pragma unroll
+        for (int q = 0; q < NI; q += 4)
+            *reinterpret_cast<float4 *>(o + q) = make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]);
+    } else {
+#pragma unroll
+        for (int q = 0; q < NI; q++) o[q] = v[q];
+    }
+}
+
+// The NI values of one column, the first ni of them real (IL: interleaved, one
+// or two vector loads).
+template <int NI, bool IL>
+__device__ __forceinline__ void load_column(float (&v)[NI], const float *__restrict__ xb, int i, long ncol, int ni) {
+    if constexpr (IL && NI % 4 == 0) {
+        const float4 *p = reinterpret_cast<const float4 *>(xb + (size_t)i * NI);
+#pragma unroll
+        for (int q = 0; q < NI / 4; q++) {
+            const float4 f = p[q];
+            v[4 * q] = f.x, v[4 * q + 1] = f.y, v[4 * q + 2] = f.z, v[4 * q + 3] = f.w;
+        }
+    } else if constexpr (IL && NI == 2) {
+        const float2 f = *reinterpret_cast<const float2 *>(xb + (size_t)i * NI);
+        v[0] = f.x, v[1] = f.y;
+    } else {
+#pragma unroll
+        for (int q = 0; q < NI; q++) v[q] = q < ni ? xb[(size_t)q * ncol + i] : 0.f;
+    }
+}
+
 // y[b][i] = sum_e M[i][e] x[b][col_e] - sum_q U[q*nrow + i] t[b][q] (+ add[b][i]).
+// IL: x is interleaved (k_interleave).  A row's columns are scattered over
+// about ten cache lines per 32 of them, and each instance's gather pays for all
+// of those; side by side, one gather serves the group (30 m, 256 instances: 222
+// -> 153 us per launch).
 // One warp takes kSpmvRows rows one after the other (the CTA's barriers, its
 // p.Ap partial and its arrival are shared by them; four entries per lane are
 // in flight); the NI sums are reduced over the warp by exchanging halves, so a
 // row costs NI + 1 shuffles instead of 5 NI.
 // grid: (ceil(nb/NI), ceil(nrow / kSpmvBlock)).
-// With dot_part: the p.Ap partials (dot_x = p) per CTA, [nb][gridDim.y], and
-// the last CTA of each instance group leaves alpha_k = (r.z)_k / p.Ap.
+// With dot_part: the p.Ap partials (dot_x = p) per CTA, [nb][gridDim.y].
 constexpr int kSpmvRows = 2;
 constexpr int kSpmvBlock = kThreads / 32 * kSpmvRows;  // rows per CTA
 
-template <int NI>
+template <int NI, bool IL>
 __global__ void __launch_bounds__(kThreads)
 k_spmv_lr(const int *__restrict__ rp, const GatherW *__restrict__ ent, int nrow, long ncol,
           const float *__restrict__ x, float *__restrict__ y, const float *__restrict__ U,
           const float *__restrict__ t, int nq, const float *__restrict__ add, const float *__restrict__ dot_x,
-          double *__restrict__ dot_part, CgScal S, int k, int nbatch, const int *__restrict__ act) {
+          double *__restrict__ dot_part, int nbatch, const int *__restrict__ act) {
     pdl_enter();
     const int b0 = blockIdx.x * NI;
     const int ni = min(NI, nbatch - b0);
@@ -140,9 +187,10 @@ k_spmv_lr(const int *__restrict__ rp, const GatherW *__restrict__ ent, int nrow,
 #pragma unroll
             for (int c = 0; c < 4; c++) {
                 if (e + 32 * c >= e1) break;
+                float v[NI];
+                load_column<NI, IL>(v, xb, g[c].i, ncol, ni);
 #pragma unroll
-                for (int q = 0; q < NI; q++)
-                    if (on[q]) acc[q] += g[c].w * xb[(size_t)q * ncol + g[c].i];
+                for (int q = 0; q < NI; q++) acc[q] += g[c].w * v[q];
             }
         }
         inst = warp_sum_many<NI>(acc);
@@ -167,18 +215,6 @@ k_spmv_lr(const int *__restrict__ rp, const GatherW *__restrict__ ent, int nrow,
 #pragma unroll
         for (int w = 0; w < kThreads / 32; w++) s += sh[w][threadIdx.x];
         dot_part[(size_t)(b0 + threadIdx.x) * gridDim.y + blockIdx.y] = s;
-    }
-    if (last_block(S.cnt + b0, gridDim.y)) {
-        if (wid < ni && !inactive(act, b0 + wid)) {
-            const int b = b0 + wid;
-            const double pap = warp_sum_fresh(dot_part + (size_t)b * gridDim.y, gridDim.y);
-            if (lane == 0) {
-                double a = S.sc[(size_t)b * S.nsc + k] / pap;
-                if (!isfinite(a)) a = 0;  // pcg.c:80-83, pcg.cu:27-30
-                S.ab[2 * b] = (float)a;
-            }
-        }
-        if (threadIdx.x == 0) S.cnt[b0] = 0;
     }
 }
 

@@ -179,14 +179,15 @@ struct Recon {
     struct CgBufs {
         float *x, *r, *p, *z, *Ap, *rhs;
         double *pap, *rr, *rz, *bb;
+        int npap;  // p.Ap partials the operator leaves per instance
         CgScal S;
     };
     // state and work buffers
     DevBuf<float> x, r, p, z, Ap, rhs, opd, grad, gin;
     DevBuf<double> tt_part, pap_part, rr_part, rz_part, bb_part, sc;
-    DevBuf<float> res, ab, tt;
+    DevBuf<float> res, be, tt;
     DevBuf<unsigned> cnt, cnt_tt;
-    CgScal scal() const { return CgScal{sc.p, nsc, ab.p, cnt.p, res.p}; }
+    CgScal scal() const { return CgScal{sc.p, nsc, be.p, cnt.p, res.p}; }
 
     // Serving: per-instance participation flags read by every kernel of the
     // step (1: run, 0: leave the instance untouched).  All ones except while a
@@ -214,9 +215,9 @@ struct Recon {
     DevBuf<float> w0_v, w1v, fwt, nwv;
     DevBuf<float> fa, fr, fp, fAp, frhs, opdf, opdw;
     DevBuf<double> w1_part, nw_part, f_pap, f_rr, f_rz, f_bb, fsc;
-    DevBuf<float> fres, fab;
+    DevBuf<float> fres, fbe;
     DevBuf<unsigned> fcnt;
-    CgScal fscal() const { return CgScal{fsc.p, fnsc, fab.p, fcnt.p, fres.p}; }
+    CgScal fscal() const { return CgScal{fsc.p, fnsc, fbe.p, fcnt.p, fres.p}; }
     // grid fit: slaving term of FitL (CSR), applied into fslv and added by k_fit_hxt
     bool has_slave = false;
     DevBuf<int> as_rp;
@@ -231,11 +232,17 @@ struct Recon {
     DevBuf<double> lr_part;
     DevBuf<float> lr_t;
     DevBuf<unsigned> lr_cnt;
-    void spmv(const DevBuf<int> &rp, const DevBuf<GatherW> &e, int nrow, long ncol, const float *xin, float *out,
-              const float *U, int nq, const float *add, double *dot, int k, cudaStream_t s);
+    void spmv(const DevBuf<int> &rp, const DevBuf<GatherW> &e, int nrow, long ncol, const float *xin, bool il,
+              float *out, const float *U, int nq, const float *add, const float *dot_x, double *dot,
+              cudaStream_t s);
     void lr_dot(const float *xin, const float *V, int nq, long n, cudaStream_t s);
     static bool cg_step_fits(long n) { return n <= 8L * 8 * kStepThreads; }
-    bool cg_step(const CgBufs &B, long n, int k, int iters, int init, const float *V, int nq, cudaStream_t s);
+    bool cg_step(const CgBufs &B, long n, int k, int iters, int init, const float *V, int nq, float *pil,
+                 cudaStream_t s);
+    // instances side by side in the vectors the fit's sparse rows gather from
+    int fit_il() const { return nb == 1 ? 1 : nb == 2 ? 2 : nb <= 4 ? 4 : 8; }
+    DevBuf<float> f_il, f_pil;  // any vector (layers or commands), and p of the CG
+    const float *interleave(const float *xin, long n, cudaStream_t s);
     void build_fit_sparse(const mb_fit_sparse_desc *f);
     void alloc_fit_state();
 
@@ -288,10 +295,10 @@ struct Recon {
     void rebuild_fdpcg_device();
     int autotune(int reps, float *ms_out);
     void pupil_rows(bool from_x, const float *xin, cudaStream_t s);
-    void hxt_rows(const float *xin, float *out, double *dot_part, int do_l2, int k, cudaStream_t s);
+    void hxt_rows(const float *xin, float *out, double *dot_part, int do_l2, cudaStream_t s);
     // the arguments of those launches (also gathered by a ReconGroup)
     PupilArgs pupil_args(bool from_x, const float *xin, int w0) const;
-    HxtArgs hxt_args(const float *xin, float *out, double *dot_part, int do_l2, int k) const;
+    HxtArgs hxt_args(const float *xin, float *out, double *dot_part, int do_l2) const;
     void build_wfs_tables(const mb_recon_desc *d);
     void build_fdpcg(const mb_fdpcg_desc *fd);
     void build_fit(const mb_fit_desc *f);
@@ -301,11 +308,17 @@ struct Recon {
     // operator pieces (enqueue on `s`)
     void op_hx(const float *xin, cudaStream_t s);
     void op_rhs(const float *g, float *out, cudaStream_t s);
-    void op_lhs(const float *xin, float *out, double *dot_part, cudaStream_t s, int k = 0);
+    void op_lhs(const float *xin, float *out, double *dot_part, cudaStream_t s);
     bool op_fdpcg(float *rin, float *zout, double *rz_part, cudaStream_t s, int k = 0, int init = 0,
                   bool in_cg = false, float *xupd = nullptr, const float *pupd = nullptr,
                   const float *Apupd = nullptr, float *pnext = nullptr);
-    bool fd_cluster = false;  // k_fd_inv<true> fits as clusters of nps CTAs
+    using FdInvKern = void (*)(const cplx *, const float *, float *, double *, FdTab, const cplx *, long, int, CgScal, int,
+                               int, const int *, float *);
+    FdInvKern fd_inv_kern(bool pu) const {  // by whether its groups hold several layers
+        return fdtab.ng < nps ? (pu ? k_fd_inv<true, true> : k_fd_inv<false, true>)
+                              : (pu ? k_fd_inv<true, false> : k_fd_inv<false, false>);
+    }
+    bool fd_cluster = false;  // k_fd_inv<true> fits as clusters of an instance's group CTAs
     // the fused preconditioner (k_fd_fused): an instance's layers split over
     // one cluster of fused_tab.C CTAs; fd_mode 1 = three kernels, 2 = fused
     bool fd_fused_ok = false;
@@ -329,13 +342,13 @@ struct Recon {
     void form_fdpcg_data(const double *neam);
     void set_fdpcg_mode(int mode);
     void enqueue_solve(cudaStream_t s);
-    using AmulFn = std::function<void(const float *, float *, double *, int)>;
+    using AmulFn = std::function<void(const float *, float *, double *)>;
     // preconditioners return true when they also left p = z + beta p
     using MmulFn = std::function<bool(float *, float *, double *, int, int)>;
     using XrMmulFn = std::function<bool(int)>;
     void enqueue_cg(const CgBufs &B, long n, int nblk, int iters, const AmulFn &Amul,
                     const MmulFn &Mmul, cudaStream_t s, const XrMmulFn &XrMmul = XrMmulFn(),
-                    const float *V = nullptr, int nq = 0);
+                    const float *V = nullptr, int nq = 0, float *pil = nullptr);
     // One CG solve taken apart at its operator applications, so that a
     // ReconGroup can apply the operator of several reconstructors in one
     // launch: after A x -> cg_init; after A p_k -> cg_post (true: done).
@@ -348,14 +361,15 @@ struct Recon {
         float *zp;
         const float *V = nullptr;  // low-rank columns whose t = V' p cg_step leaves for the next A p
         int nq = 0;
+        float *pil = nullptr;  // where cg_step leaves p interleaved
     };
     void cg_init(CgRun &c, int k, cudaStream_t s);
     bool cg_post(CgRun &c, int k, cudaStream_t s);
     CgRun solve_run(cudaStream_t s);  // the tomography CG (its preconditioner launched on s)
     void op_rhs_gp(const float *g, cudaStream_t s);  // the first launch of op_rhs (gradient weighting)
     void op_fitR(const float *xin, float *out, cudaStream_t s);
-    // t_ready: V' ain is already in lr_t (left by cg_step)
-    void op_fitL(const float *ain, float *out, double *dot_part, cudaStream_t s, int k = 0, bool t_ready = false);
+    // ready: V' ain and ain interleaved are already there (left by cg_step)
+    void op_fitL(const float *ain, float *out, double *dot_part, cudaStream_t s, bool ready = false);
     void enqueue_fit(cudaStream_t s);
     void time_stages(int reps, float *ms, double *bytes, int *launches);
     void capture_graph();
@@ -694,15 +708,14 @@ void Recon::pupil_rows(bool from_x, const float *xin, cudaStream_t s) {
     }
 }
 
-HxtArgs Recon::hxt_args(const float *xin, float *out, double *dot_part, int do_l2, int k) const {
-    return HxtArgs{obuf.p, xin,     out,   dot_part, HxtIndex{hxt_x0.p, hxt_xw.p, hxt_y0.p, hxt_yw.p},
-                   hxttab, laytab,  nps,   nwfs,     orows,
-                   ostride, nxtot,  do_l2, scal(),   k,
-                   act()};
+HxtArgs Recon::hxt_args(const float *xin, float *out, double *dot_part, int do_l2) const {
+    return HxtArgs{obuf.p, xin,    out, dot_part, HxtIndex{hxt_x0.p, hxt_xw.p, hxt_y0.p, hxt_yw.p},
+                   hxttab, laytab, nps, nwfs,     orows,
+                   ostride, nxtot, do_l2, act()};
 }
 
-void Recon::hxt_rows(const float *xin, float *out, double *dot_part, int do_l2, int k, cudaStream_t s) {
-    launch(hxt_kern(hrows), dim3(nblk_hxt, nb), dim3(kHxtThreads), 0, s, hxt_args(xin, out, dot_part, do_l2, k));
+void Recon::hxt_rows(const float *xin, float *out, double *dot_part, int do_l2, cudaStream_t s) {
+    launch(hxt_kern(hrows), dim3(nblk_hxt, nb), dim3(kHxtThreads), 0, s, hxt_args(xin, out, dot_part, do_l2));
 }
 
 void Recon::build_wfs_tables(const mb_recon_desc *d) {
@@ -1029,37 +1042,70 @@ void Recon::build_fdpcg(const mb_fdpcg_desc *fd) {
             if (F.px < 0 && kFftPairs[i][0] * kFftPairs[i][1] == F.nx) F.px = i;
             if (F.py < 0 && kFftPairs[i][0] * kFftPairs[i][1] == F.ny) F.py = i;
         }
-        fd_bufn = std::max(fd_bufn, std::max(F.ny / 2 * F.nx, F.ny * (F.nx / 2 + 1)));
-        if (F.px >= 0) fd_bufn = std::max(fd_bufn, fft2_scratch(F.px, true, F.ny / 2));
-        if (F.py >= 0) fd_bufn = std::max(fd_bufn, fft2_scratch(F.py, false, F.nx / 2 + 1));
         twn = std::max(twn, F.nx + F.ny);
     }
+    // The inverse's groups: equal layers together, up to the points (and a CTA's
+    // columns) of the largest layer, once an instance's CTAs no longer run all
+    // at once.  Its cluster then holds CTAs of equal work: with one layer each,
+    // the small layers' CTAs kept their places on the SMs until the largest's
+    // were done (30 m, 256 instances: 91 -> 70 us).  While all CTAs are resident
+    // a group only lengthens the chain (6 instances: 12.4 -> 16 us).  Each layer
+    // alone, too, where the groups' buffers would leave fewer CTAs on an SM.
+    auto buffers = [&](long limit) {
+        fdtab.ng = fd_bufn = 0;
+        for (int l = 0; l < nps; l++) {
+            const FdLayer &F = fl[l];
+            int g = 0;
+            for (; g < fdtab.ng; g++) {
+                const FdGroup &Q = fdtab.g[g];
+                if (fl[Q.l[0]].nx == F.nx && fl[Q.l[0]].ny == F.ny && (Q.n + 1L) * F.nx * F.ny <= limit &&
+                    (Q.n + 1) * (F.nx / 2 + 1) <= kFftThreads)
+                    break;
+            }
+            if (g == fdtab.ng) fdtab.g[fdtab.ng++] = FdGroup{};
+            fdtab.g[g].l[fdtab.g[g].n++] = (signed char)l;
+        }
+        for (int g = 0; g < fdtab.ng; g++) {
+            const FdLayer &F = fl[fdtab.g[g].l[0]];
+            const int n = fdtab.g[g].n;
+            fd_bufn = std::max(fd_bufn, n * std::max(F.ny / 2 * F.nx, F.ny * (F.nx / 2 + 1)));
+            if (F.px >= 0) fd_bufn = std::max(fd_bufn, fft2_scratch(F.px, true, n * F.ny / 2));
+            if (F.py >= 0) fd_bufn = std::max(fd_bufn, fft2_scratch(F.py, false, n * (F.nx / 2 + 1)));
+        }
+        return (2 * (size_t)fd_bufn + twn) * sizeof(cplx);
+    };
+    long most = 0;
+    for (const FdLayer &F : fl) most = std::max(most, (long)F.nx * F.ny);
+    constexpr size_t kSmSmem = 227 * 1024, kPerCta = 1024;
+    const size_t alone = buffers(0);
+    fd_smem = (long)nb * nps > 2 * 148 ? buffers(most) : alone;
+    if (fd_smem > 200 * 1024 || kSmSmem / (fd_smem + kPerCta) < std::min<size_t>(2, kSmSmem / (alone + kPerCta)))
+        fd_smem = buffers(0);
     fd_lay.upload(fl);
     for (int l = 0; l < nps; l++) fdtab.l[l] = fl[l];
     fd_tw.upload(tw);
-    fd_smem = (2 * (size_t)fd_bufn + twn) * sizeof(cplx);
     MB_REQUIRE(fd_smem <= 200 * 1024, "fdpcg: layer FFT needs %zu bytes of shared memory", fd_smem);
     MB_CUDA_TRY(cudaFuncSetAttribute(k_fd_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fd_smem));
-    MB_CUDA_TRY(cudaFuncSetAttribute(k_fd_inv<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fd_smem));
-    MB_CUDA_TRY(cudaFuncSetAttribute(k_fd_inv<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fd_smem));
-    // the CG step's inverse runs as clusters of the nps layer CTAs of an instance when such a cluster fits
+    for (bool pu : {false, true})
+        MB_CUDA_TRY(cudaFuncSetAttribute(fd_inv_kern(pu), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fd_smem));
+    // the CG step's inverse runs as clusters of the group CTAs of an instance when such a cluster fits
     fd_cluster = false;
-    if (nps <= 16) {
-        if (nps > 8)
-            MB_CUDA_TRY(cudaFuncSetAttribute(k_fd_inv<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    if (fdtab.ng <= 16) {
+        if (fdtab.ng > 8)
+            MB_CUDA_TRY(cudaFuncSetAttribute(fd_inv_kern(true), cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = (unsigned)nps;
+        at[0].val.clusterDim.x = (unsigned)fdtab.ng;
         at[0].val.clusterDim.y = 1;
         at[0].val.clusterDim.z = 1;
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(nps, nb);
+        cfg.gridDim = dim3(fdtab.ng, nb);
         cfg.blockDim = dim3(kFftThreads);
         cfg.dynamicSmemBytes = fd_smem;
         cfg.attrs = at;
         cfg.numAttrs = 1;
         int ncl = 0;
-        fd_cluster = cudaOccupancyMaxActiveClusters(&ncl, k_fd_inv<true>, &cfg) == cudaSuccess && ncl > 0;
+        fd_cluster = cudaOccupancyMaxActiveClusters(&ncl, fd_inv_kern(true), &cfg) == cudaSuccess && ncl > 0;
         cudaGetLastError();  // a size the device refuses only means the unclustered path
         if (const char *e = std::getenv("MAOS_B200_FD_CLUSTER")) fd_cluster = fd_cluster && e[0] != '0';
     }
@@ -1197,6 +1243,12 @@ void Recon::build_fdpcg_fused(const std::vector<FdIndex> &idx, const std::vector
     fd_mem.upload(mem);
     fused_tab = T;
     fd_fused_ok = true;
+    // the fused form while every instance's cluster runs at once beside the
+    // others: 6 instances of the 30 m system 314 against 364 us per step of 4
+    // iterations, 8 (two rounds of clusters) 373 against 379; 5 of the 39 m one
+    // 569 against 636, 8 731 against 706.  mb_autotune and mb_fdpcg_mode choose
+    // otherwise.
+    if (nb * fused_tab.C <= 96) fd_mode = 2;
 }
 
 // The data term's geometry on the device: per block its base pupil
@@ -1382,7 +1434,7 @@ void Recon::build(const mb_recon_desc *d) {
     bb_part.alloc((size_t)nb * nblk_x);
     sc.alloc((size_t)nb * nsc);
     res.alloc(nb);
-    ab.alloc((size_t)nb * 2);
+    be.alloc(nb);
     tt.alloc((size_t)nb * nwfs * 2);
     cnt.alloc(nb);
     cnt_tt.alloc((size_t)nb * nwfs);
@@ -1400,7 +1452,7 @@ void Recon::build(const mb_recon_desc *d) {
     gin.zero_async(stream);
     sc.zero_async(stream);
     res.zero_async(stream);
-    ab.zero_async(stream);
+    be.zero_async(stream);
     tt.zero_async(stream);
     cnt.zero_async(stream);
     cnt_tt.zero_async(stream);
@@ -1425,10 +1477,10 @@ void Recon::op_rhs(const float *g, float *out, cudaStream_t s) {
     // TomoR: x = Hx^T GP^T NEA^-1 (I - TT PTT) g   (recon_utils.c:397, tomo.cu:607)
     op_rhs_gp(g, s);
     pupil_rows(false, nullptr, s);
-    hxt_rows(nullptr, out, nullptr, 0, 0, s);
+    hxt_rows(nullptr, out, nullptr, 0, s);
 }
 
-void Recon::op_lhs(const float *xin, float *out, double *dot_part, cudaStream_t s, int k) {
+void Recon::op_lhs(const float *xin, float *out, double *dot_part, cudaStream_t s) {
     // TomoL: Hx^T GP^T NEA^-1 (I - TT PTT) GP Hx x + L2^T L2 x   (recon_utils.c:447, tomo.cu:639)
     if (split) {  // no tip/tilt term: Hx, GP, NEA, GP^T fused per pupil-row block
         pupil_rows(true, xin, s);
@@ -1438,7 +1490,7 @@ void Recon::op_lhs(const float *xin, float *out, double *dot_part, cudaStream_t 
                                                           nwfs, nxp, np, ngrad, 1, tt.p, cnt_tt.p, act());
         pupil_rows(false, nullptr, s);
     }
-    hxt_rows(xin, out, dot_part, 1, k, s);
+    hxt_rows(xin, out, dot_part, 1, s);
 }
 
 // The block solve of every (half-spectrum block, instance), fd_mul_ni
@@ -1458,20 +1510,20 @@ bool Recon::op_fdpcg(float *rin, float *zout, double *rzp, cudaStream_t s, int k
     // on the half spectrum as in cuda/fdpcg.cu (fdpcg_mul_block_sync_half)
     if (in_cg && pnext && fd_mode == 2) {  // one launch: layers split over an instance's cluster
         launch_cluster(k_fd_fused, dim3(fused_tab.C, nb), dim3(kFusedThreads), fd_fsmem, s, fused_tab.C, rin, fdtab,
-                       fused_tab, fd_tw.p, fd_M.p, fd_mem.p, fd_bs, nxtot, xupd, Apupd, scal(), k, init, act(),
-                       pnext);
+                       fused_tab, fd_tw.p, fd_M.p, fd_mem.p, fd_bs, nxtot, xupd, Apupd,
+                       PapParts{pap_part.p, nblk_hxt}, scal(), k, init, act(), pnext);
         return true;
     }
     launch(k_fd_fwd, dim3(nps, nb), dim3(kFftThreads), fd_smem, s, rin, spec.p, fdtab, fd_tw.p, nxtot, fd_bufn, xupd,
-                                                        pupd, Apupd, xupd ? ab.p : nullptr, act());
+           pupd, Apupd, PapParts{pap_part.p, nblk_hxt}, scal(), k, act());
     fd_mul(s);
     CgScal S = in_cg ? scal() : CgScal{};
     if (in_cg && pnext && fd_cluster) {  // the p update inside, clusters of the layer CTAs
-        launch_cluster(k_fd_inv<true>, dim3(nps, nb), dim3(kFftThreads), fd_smem, s, nps, spec2.p, rin, zout, rzp,
-                       fdtab, fd_tw.p, nxtot, fd_bufn, S, k, init, act(), pnext);
+        launch_cluster(fd_inv_kern(true), dim3(fdtab.ng, nb), dim3(kFftThreads), fd_smem, s, fdtab.ng, spec2.p, rin, zout,
+                       rzp, fdtab, fd_tw.p, nxtot, fd_bufn, S, k, init, act(), pnext);
         return true;
     }
-    launch(k_fd_inv<false>, dim3(nps, nb), dim3(kFftThreads), fd_smem, s, spec2.p, rin, zout, rzp, fdtab, fd_tw.p,
+    launch(fd_inv_kern(false), dim3(fdtab.ng, nb), dim3(kFftThreads), fd_smem, s, spec2.p, rin, zout, rzp, fdtab, fd_tw.p,
            nxtot, fd_bufn, S, k, init, act(), (float *)nullptr);
     return false;
 }
@@ -1479,7 +1531,7 @@ bool Recon::op_fdpcg(float *rin, float *zout, double *rzp, cudaStream_t s, int k
 void Recon::cg_init(CgRun &c, int k, cudaStream_t s) {
     // after Ap = A x: r = b - A x, b.b, z = M r, (r.z)_k, p = z
     const CgBufs &B = c.B;
-    if (!c.Mmul && cg_step(B, c.n, k, c.iters, 1, c.V, c.nq, s)) return;
+    if (!c.Mmul && cg_step(B, c.n, k, c.iters, 1, c.V, c.nq, c.pil, s)) return;
     launch(k_cg_init_r, dim3(c.nblk, nb), dim3(kThreads), 0, s, B.rhs, B.Ap, B.r, B.bb, c.n, B.S, c.iters, act());
     bool pdone = false;
     if (c.Mmul) {
@@ -1493,15 +1545,15 @@ void Recon::cg_init(CgRun &c, int k, cudaStream_t s) {
 }
 
 bool Recon::cg_post(CgRun &c, int k, cudaStream_t s) {
-    // after Ap = A p_k (whose last block left alpha_k)
+    // after Ap = A p_k and the p.Ap partials
     const CgBufs &B = c.B;
-    if (!c.Mmul && cg_step(B, c.n, k, c.iters, 0, c.V, c.nq, s)) return k + 1 == c.iters;
+    if (!c.Mmul && cg_step(B, c.n, k, c.iters, 0, c.V, c.nq, c.pil, s)) return k + 1 == c.iters;
     bool pdone;
     if (c.XrMmul && k + 1 < c.iters) {
         pdone = c.XrMmul(k);  // x, r update and preconditioner; beta_k (and p, when it says so)
     } else {
-        launch(k_cg_update_xr, dim3(c.nblk, nb), dim3(kThreads), 0, s, B.x, B.r, B.p, B.Ap, B.rr, c.n, B.S, k,
-               c.iters, c.Mmul ? 0 : 1, act());
+        launch(k_cg_update_xr, dim3(c.nblk, nb), dim3(kThreads), 0, s, B.x, B.r, B.p, B.Ap, B.rr, c.n,
+               PapParts{B.pap, B.npap}, B.S, k, c.iters, c.Mmul ? 0 : 1, act());
         if (k + 1 == c.iters) return true;
         pdone = c.Mmul ? c.Mmul(B.r, B.z, B.rz, k, 0) : false;  // beta_k (and p, when it says so)
     }
@@ -1515,12 +1567,13 @@ bool Recon::cg_post(CgRun &c, int k, cudaStream_t s) {
 // false where an instance's vector does not fit a cluster's registers (8
 // elements per thread of 8 CTAs; then the separate kernels run).  As few CTAs
 // as keep 4 elements per thread.
-bool Recon::cg_step(const CgBufs &B, long n, int k, int iters, int init, const float *V, int nq, cudaStream_t s) {
+bool Recon::cg_step(const CgBufs &B, long n, int k, int iters, int init, const float *V, int nq, float *pil,
+                    cudaStream_t s) {
     if (!cg_step_fits(n)) return false;
     const int C = (int)std::min(8L, (n + 4L * kStepThreads - 1) / (4L * kStepThreads));
     const auto kern = n <= 4L * kStepThreads * C ? k_cg_step<4> : k_cg_step<8>;
     launch_cluster(kern, dim3(C, nb), dim3(kStepThreads), 0, s, C, B.x, B.r, B.p, (const float *)B.Ap,
-                   (const float *)B.rhs, n, B.S, k, iters, init, V, nq, lr_t.p, act());
+                   (const float *)B.rhs, n, PapParts{B.pap, B.npap}, B.S, k, iters, init, V, nq, lr_t.p, pil, fit_il(), act());
     return true;
 }
 
@@ -1532,24 +1585,25 @@ bool Recon::cg_step(const CgBufs &B, long n, int k, int iters, int init, const f
 // XrMmul, when given, performs the x/r update of a non-final iteration
 // together with the preconditioner.
 void Recon::enqueue_cg(const CgBufs &B, long n, int nblk, int iters, const AmulFn &Amul,
-                       const MmulFn &Mmul, cudaStream_t s, const XrMmulFn &XrMmul, const float *V, int nq) {
-    CgRun c{B, n, nblk, iters, Mmul, XrMmul, Mmul ? B.z : B.r, V, nq};
-    Amul(B.x, B.Ap, nullptr, 0);
+                       const MmulFn &Mmul, cudaStream_t s, const XrMmulFn &XrMmul, const float *V, int nq,
+                       float *pil) {
+    CgRun c{B, n, nblk, iters, Mmul, XrMmul, Mmul ? B.z : B.r, V, nq, pil};
+    Amul(B.x, B.Ap, nullptr);
     cg_init(c, 0, s);
     for (int k = 0; k < iters; k++) {
         if (k > 0 && k % kCgRestart == 0) {
             // restart as lib/pcg.c:61 does every 100 iterations: r = b - A x,
             // z = M r, p = z, (r.z)_k afresh (the p of the previous step is dropped)
-            Amul(B.x, B.Ap, nullptr, 0);
+            Amul(B.x, B.Ap, nullptr);
             cg_init(c, k, s);
         }
-        Amul(B.p, B.Ap, B.pap, k);  // its last block leaves alpha_k
+        Amul(B.p, B.Ap, B.pap);
         if (cg_post(c, k, s)) break;
     }
 }
 
 Recon::CgRun Recon::solve_run(cudaStream_t s) {
-    CgRun c{CgBufs{x.p, r.p, p.p, z.p, Ap.p, rhs.p, pap_part.p, rr_part.p, rz_part.p, bb_part.p, scal()},
+    CgRun c{CgBufs{x.p, r.p, p.p, z.p, Ap.p, rhs.p, pap_part.p, rr_part.p, rz_part.p, bb_part.p, nblk_hxt, scal()},
             nxtot, nblk_x, maxit, MmulFn(), XrMmulFn(), r.p};
     if (precond) {
         c.Mmul = [this, s](float *in, float *out, double *dot, int k, int init) {
@@ -1565,24 +1619,35 @@ Recon::CgRun Recon::solve_run(cudaStream_t s) {
 void Recon::enqueue_solve(cudaStream_t s) {
     op_rhs(gin.p, rhs.p, s);
     CgRun c = solve_run(s);
-    AmulFn A = [&](const float *in, float *out, double *dot, int k) { op_lhs(in, out, dot, s, k); };
+    AmulFn A = [&](const float *in, float *out, double *dot) { op_lhs(in, out, dot, s); };
     enqueue_cg(c.B, c.n, c.nblk, c.iters, A, c.Mmul, s, c.XrMmul);
 }
 
 // y = M x - U (V'x) for all instances: one warp per row, NI instances per CTA.
-void Recon::spmv(const DevBuf<int> &rp, const DevBuf<GatherW> &e, int nrow, long ncol, const float *xin, float *out,
-                 const float *U, int nq, const float *add, double *dot, int k, cudaStream_t s) {
+// xin: interleaved over fit_il() instances (il), or instance-major.
+void Recon::spmv(const DevBuf<int> &rp, const DevBuf<GatherW> &e, int nrow, long ncol, const float *xin, bool il,
+                 float *out, const float *U, int nq, const float *add, const float *dot_x, double *dot,
+                 cudaStream_t s) {
     const unsigned ry = (unsigned)((nrow + kSpmvBlock - 1) / kSpmvBlock);
-    const CgScal S = dot ? fscal() : CgScal{};
-    const float *dx = dot ? xin : nullptr;
-#define MB_SPMV(NI)                                                                                            \
-    launch(k_spmv_lr<NI>, dim3((unsigned)((nb + NI - 1) / NI), ry), dim3(kThreads), 0, s, rp.p, e.p, nrow, ncol, \
-           xin, out, U, lr_t.p, nq, add, dx, dot, S, k, nb, act())
-    if (nb == 1) MB_SPMV(1);
-    else if (nb == 2) MB_SPMV(2);
-    else if (nb <= 4) MB_SPMV(4);
-    else MB_SPMV(8);
-#undef MB_SPMV
+    const float *dx = dot ? dot_x : nullptr;
+    using K = void (*)(const int *, const GatherW *, int, long, const float *, float *, const float *, const float *,
+                       int, const float *, const float *, double *, int, const int *);
+    const int ni = fit_il();
+    const K kern = ni == 1   ? k_spmv_lr<1, true>
+                   : ni == 2 ? (il ? k_spmv_lr<2, true> : k_spmv_lr<2, false>)
+                   : ni == 4 ? (il ? k_spmv_lr<4, true> : k_spmv_lr<4, false>)
+                             : (il ? k_spmv_lr<8, true> : k_spmv_lr<8, false>);
+    launch(kern, dim3((unsigned)((nb + ni - 1) / ni), ry), dim3(kThreads), 0, s, rp.p, e.p, nrow, ncol, xin, out, U,
+           lr_t.p, nq, add, dx, dot, nb, act());
+}
+
+// xin [nb][n] with fit_il() instances side by side.
+const float *Recon::interleave(const float *xin, long n, cudaStream_t s) {
+    const int ni = fit_il();
+    if (ni == 1) return xin;
+    const auto kern = ni == 2 ? k_interleave<2> : ni == 4 ? k_interleave<4> : k_interleave<8>;
+    launch(kern, dim3(nblocks(n), (nb + ni - 1) / ni), dim3(kThreads), 0, s, xin, f_il.p, n, nb);
+    return f_il.p;
 }
 
 // t[b][q] = V_q' x_b (FP64 partials, fixed-order total)
@@ -1603,7 +1668,8 @@ void Recon::lr_dot(const float *xin, const float *V, int nq, long n, cudaStream_
 void Recon::op_fitR(const float *xin, float *out, cudaStream_t s) {
     if (fit_sparse) {
         if (nfr) lr_dot(xin, frv.p, nfr, nxtot, s);
-        spmv(frm_rp, frm_e, (int)nact, nxtot, xin, out, nfr ? fru.p : nullptr, nfr, nullptr, nullptr, 0, s);
+        spmv(frm_rp, frm_e, (int)nact, nxtot, interleave(xin, nxtot, s), true, out, nfr ? fru.p : nullptr, nfr, nullptr,
+             nullptr, nullptr, s);
         return;
     }
     launch(nps <= 8 ? k_hx<8> : k_hx<16>, dim3(nblk_f, nfit, nb), dim3(kThreads), 0, s, xin, opdf.p, hxp.fwd.p, laytab, nps, nfit, nfx, nfy,
@@ -1611,16 +1677,17 @@ void Recon::op_fitR(const float *xin, float *out, cudaStream_t s) {
     launch(k_fit_w, dim3(nblk_f, nfit, nb), dim3(kThreads), 0, s, opdf.p, opdw.p, w0_rp.p, w0_ci.p, w0_v.p, w1v.p,
                                                        fwt.p, w1_part.p, nblk_f, nf, nfit, act());
     launch(k_fit_hxt, dim3(nblk_a, nb), dim3(kThreads), 0, s, opdw.p, nullptr, out, nullptr, fitpad(), dmtab, ndm,
-           nfit, nfx, nfy, nact, LowRank{}, fscal(), 0, (const float *)nullptr, act());
+           nfit, nfx, nfy, nact, LowRank{}, (const float *)nullptr, act());
 }
 
 // FitL: sum_f wt_f HA_f^T (W0 - W1 W1^T) HA_f a + NW NW^T a + actslave a
 //       (recon_utils.c:536, fit.cu:213-235)
 // assembled: FL.M a - FL.U (FL.V' a)                 (lib/muv.c:37, solve.cu:36)
-void Recon::op_fitL(const float *ain, float *out, double *dot_part, cudaStream_t s, int k, bool t_ready) {
+void Recon::op_fitL(const float *ain, float *out, double *dot_part, cudaStream_t s, bool ready) {
     if (fit_sparse) {
-        if (nfl && !t_ready) lr_dot(ain, flv.p, nfl, nact, s);
-        spmv(flm_rp, flm_e, (int)nact, nact, ain, out, nfl ? flu.p : nullptr, nfl, nullptr, dot_part, k, s);
+        if (nfl && !ready) lr_dot(ain, flv.p, nfl, nact, s);
+        const float *ail = !ready ? interleave(ain, nact, s) : nb == 1 ? ain : f_pil.p;
+        spmv(flm_rp, flm_e, (int)nact, nact, ail, true, out, nfl ? flu.p : nullptr, nfl, nullptr, ain, dot_part, s);
         return;
     }
     LowRank lr{};
@@ -1629,23 +1696,25 @@ void Recon::op_fitL(const float *ain, float *out, double *dot_part, cudaStream_t
         lr = LowRank{nwv.p, nw_part.p, nnw, nblk_a};
     }
     if (has_slave)
-        spmv(as_rp, as_e, (int)nact, nact, ain, fslv.p, nullptr, 0, nullptr, nullptr, 0, s);
+        spmv(as_rp, as_e, (int)nact, nact, ain, false, fslv.p, nullptr, 0, nullptr, nullptr, nullptr, s);
     launch(ndm <= 8 ? k_hx<8> : k_hx<16>, dim3(nblk_f, nfit, nb), dim3(kThreads), 0, s, ain, opdf.p, ha.fwd.p, dmtab, ndm, nfit, nfx, nfy,
                                                     nact, w1v.p, w1_part.p, act());
     launch(k_fit_w, dim3(nblk_f, nfit, nb), dim3(kThreads), 0, s, opdf.p, opdw.p, w0_rp.p, w0_ci.p, w0_v.p, w1v.p,
                                                        fwt.p, w1_part.p, nblk_f, nf, nfit, act());
     launch(k_fit_hxt, dim3(nblk_a, nb), dim3(kThreads), 0, s, opdw.p, ain, out, dot_part, fitpad(), dmtab, ndm,
-           nfit, nfx, nfy, nact, lr, fscal(), k, has_slave ? (const float *)fslv.p : nullptr, act());
+           nfit, nfx, nfy, nact, lr, has_slave ? (const float *)fslv.p : nullptr, act());
 }
 
 // The DM fit of one step: RHS from the tomography solution, then CG warm-
 // started from the previous commands (curecon_t::fit, cuda/recon.cu:277).
 void Recon::enqueue_fit(cudaStream_t s) {
     op_fitR(x.p, frhs.p, s);
-    CgBufs B{fa.p, fr.p, fp.p, fr.p, fAp.p, frhs.p, f_pap.p, f_rr.p, f_rz.p, f_bb.p, fscal()};
-    const bool lr = fit_sparse && nfl && cg_step_fits(nact);
-    AmulFn A = [&](const float *in, float *out, double *dot, int k) { op_fitL(in, out, dot, s, k, lr && in == fp.p); };
-    enqueue_cg(B, nact, nblk_a, fit_maxit, A, MmulFn(), s, XrMmulFn(), lr ? flv.p : nullptr, lr ? nfl : 0);
+    CgBufs B{fa.p, fr.p, fp.p, fr.p, fAp.p, frhs.p, f_pap.p, f_rr.p, f_rz.p, f_bb.p,
+             fit_sparse ? nrb_a : nblk_a, fscal()};
+    const bool step = fit_sparse && cg_step_fits(nact);
+    AmulFn A = [&](const float *in, float *out, double *dot) { op_fitL(in, out, dot, s, step && in == fp.p); };
+    enqueue_cg(B, nact, nblk_a, fit_maxit, A, MmulFn(), s, XrMmulFn(), step ? flv.p : nullptr, step ? nfl : 0,
+               step && nb > 1 ? f_pil.p : nullptr);
 }
 
 // CSC (the reference's dsp) -> CSR rows of (column, value) pairs.
@@ -1686,12 +1755,12 @@ void Recon::alloc_fit_state() {
     f_rz.alloc((size_t)nb * nblk_a); f_bb.alloc((size_t)nb * nblk_a);
     fsc.alloc((size_t)nb * fnsc);
     fres.alloc(nb);
-    fab.alloc((size_t)nb * 2);
+    fbe.alloc(nb);
     fcnt.alloc(nb);
     fa.zero_async(stream);
     fsc.zero_async(stream);
     fres.zero_async(stream);
-    fab.zero_async(stream);
+    fbe.zero_async(stream);
     fcnt.zero_async(stream);
 }
 
@@ -1728,6 +1797,13 @@ void Recon::build_fit_sparse(const mb_fit_sparse_desc *f) {
         upload_f32(flv, f->flv, (size_t)nact * nfl);
     }
     lr_part.alloc((size_t)nb * kMaxLr * std::max(nblocks(nxtot), nblocks(nact)));
+    if (const int ni = fit_il(); ni > 1) {  // whole groups; the places past the last instance stay zero
+        const size_t rows = (size_t)((nb + ni - 1) / ni) * ni;
+        f_il.alloc(rows * std::max(nxtot, nact));
+        f_pil.alloc(rows * nact);
+        f_il.zero_async(stream);
+        f_pil.zero_async(stream);
+    }
     lr_t.alloc((size_t)nb * kMaxLr);
     lr_cnt.alloc(nb);
     lr_t.zero_async(stream);
@@ -1910,10 +1986,10 @@ void Recon::time_stages(int reps, float *ms, double *bytes, int *launches) {
         auto run_stage = [&]() {
             switch (st) {
                 case 0: pupil_rows(true, p.p, stream); break;
-                case 1: hxt_rows(p.p, Ap.p, pap_part.p, 1, 0, stream); break;
+                case 1: hxt_rows(p.p, Ap.p, pap_part.p, 1, stream); break;
                 case 2:
                     launch(k_cg_update_xr, dim3(nblk_x, nb), dim3(kThreads), 0, stream, z.p, rhs.p, p.p, Ap.p,
-                           rr_part.p, nxtot, scal(), 0, maxit, 0, act());
+                           rr_part.p, nxtot, PapParts{pap_part.p, nblk_hxt}, scal(), 0, maxit, 0, act());
                     break;
                 case 3:
                     launch(k_cg_update_p, dim3(nblocks((nxtot + kUpdP - 1) / kUpdP), nb), dim3(kThreads), 0,
@@ -1921,21 +1997,21 @@ void Recon::time_stages(int reps, float *ms, double *bytes, int *launches) {
                     break;
                 case 4:
                     launch(k_fd_fwd, dim3(nps, nb), dim3(kFftThreads), fd_smem, stream, rhs.p, spec.p, fdtab,
-                           fd_tw.p, nxtot, fd_bufn, z.p, p.p, Ap.p, ab.p, act());
+                           fd_tw.p, nxtot, fd_bufn, z.p, p.p, Ap.p, PapParts{pap_part.p, nblk_hxt}, scal(), 0, act());
                     break;
                 case 5: fd_mul(stream); break;
                 case 7:  // fused: scratch vectors (rhs as r, z as x, Ap, rhs as p)
                     launch_cluster(k_fd_fused, dim3(fused_tab.C, nb), dim3(kFusedThreads), fd_fsmem, stream,
                                    fused_tab.C, rhs.p, fdtab, fused_tab, fd_tw.p, fd_M.p, fd_mem.p, fd_bs, nxtot,
-                                   z.p, Ap.p, scal(), 0, 0, act(), z.p);
+                                   z.p, Ap.p, PapParts{pap_part.p, nblk_hxt}, scal(), 0, 0, act(), z.p);
                     break;
                 case 6:
                     if (pin)
-                        launch_cluster(k_fd_inv<true>, dim3(nps, nb), dim3(kFftThreads), fd_smem, stream, nps,
+                        launch_cluster(fd_inv_kern(true), dim3(fdtab.ng, nb), dim3(kFftThreads), fd_smem, stream, fdtab.ng,
                                        spec2.p, r.p, z.p, rz_part.p, fdtab, fd_tw.p, nxtot, fd_bufn, scal(), 0, 0,
                                        act(), rhs.p);
                     else
-                        launch(k_fd_inv<false>, dim3(nps, nb), dim3(kFftThreads), fd_smem, stream, spec2.p, r.p,
+                        launch(fd_inv_kern(false), dim3(fdtab.ng, nb), dim3(kFftThreads), fd_smem, stream, spec2.p, r.p,
                                z.p, rz_part.p, fdtab, fd_tw.p, nxtot, fd_bufn, CgScal{}, 0, 0, act(),
                                (float *)nullptr);
                     break;
@@ -2236,7 +2312,7 @@ struct ReconGroup {
         }
     }
     void hxt_rows(const std::vector<int> &who, const std::vector<const float *> &xin, const std::vector<float *> &out,
-                  const std::vector<double *> &dot, int do_l2, int k, cudaStream_t s) {
+                  const std::vector<double *> &dot, int do_l2, cudaStream_t s) {
         for (int rt : {1, 2, 4}) {
             std::vector<int> b;
             for (int i : who)
@@ -2248,7 +2324,7 @@ struct ReconGroup {
                 for (int e = 0; e < g.n; e++) {
                     const int i = b[c0 + e];
                     const Recon &R = *m[i];
-                    g.a[e] = R.hxt_args(xin[i], out[i], dot[i], do_l2, k);
+                    g.a[e] = R.hxt_args(xin[i], out[i], dot[i], do_l2);
                     g.grid[e] = make_uint3((unsigned)R.nblk_hxt, (unsigned)R.nb, 1u);
                     g.start[e + 1] = g.start[e] + g.grid[e].x * g.grid[e].y;
                 }
@@ -2258,15 +2334,15 @@ struct ReconGroup {
     }
     // A p for every member (TomoL): grouped where the tip/tilt split allows
     void lhs(const std::vector<const float *> &xin, const std::vector<float *> &out, const std::vector<double *> &dot,
-             int k, cudaStream_t s) {
+             cudaStream_t s) {
         std::vector<int> who;
         for (int i : order) {
             if (m[i]->split) who.push_back(i);
-            else m[i]->op_lhs(xin[i], out[i], dot[i], s, k);
+            else m[i]->op_lhs(xin[i], out[i], dot[i], s);
         }
         if (who.empty()) return;
         pupil_rows(true, who, xin, s);
-        hxt_rows(who, xin, out, dot, 1, k, s);
+        hxt_rows(who, xin, out, dot, 1, s);
     }
     void enqueue(cudaStream_t s) {
         const int n = (int)m.size();
@@ -2286,23 +2362,23 @@ struct ReconGroup {
         for (int i = 0; i < n; i++) m[i]->op_rhs_gp(m[i]->gin.p, side[i]);
         join(s);
         pupil_rows(false, all, none, s);
-        hxt_rows(all, none, rhs, nod, 0, 0, s);
+        hxt_rows(all, none, rhs, nod, 0, s);
         // CG from the warm start, iteration by iteration
         std::vector<Recon::CgRun> run;
         for (int i = 0; i < n; i++) run.push_back(m[i]->solve_run(side[i]));
         std::vector<bool> done(n, false);
-        lhs(xs, Ap, nod, 0, s);
+        lhs(xs, Ap, nod, s);
         fork(s);
         for (int i = 0; i < n; i++) m[i]->cg_init(run[i], 0, side[i]);
         join(s);
         for (int k = 0; k < maxit; k++) {
             if (k > 0 && k % kCgRestart == 0) {
-                lhs(xs, Ap, nod, 0, s);
+                lhs(xs, Ap, nod, s);
                 fork(s);
                 for (int i = 0; i < n; i++) m[i]->cg_init(run[i], k, side[i]);
                 join(s);
             }
-            lhs(ps, Ap, pap, k, s);
+            lhs(ps, Ap, pap, s);
             fork(s);
             for (int i = 0; i < n; i++)
                 if (!done[i]) done[i] = m[i]->cg_post(run[i], k, side[i]);

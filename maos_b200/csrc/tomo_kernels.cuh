@@ -121,13 +121,13 @@ __device__ __forceinline__ double warp_sum_partials(const double *part, int n) {
 }
 
 // Per-CG scalar state, per instance.  sc holds r.z of every iteration
-// (0..iters), b.b at iters+1 and the final residual at iters+2; ab the alpha
-// and beta of the current iteration; cnt the arrival counters of the
-// last-block reductions (zero between kernels).
+// (0..iters), b.b at iters+1 and the final residual at iters+2; be the beta of
+// the current iteration; cnt the arrival counters of the last-block reductions
+// (zero between kernels).
 struct CgScal {
     double *sc;
     int nsc;
-    float *ab;       // [nb][2]
+    float *be;       // [nb]
     unsigned *cnt;   // [nb]
     float *res;      // [nb]
 };
@@ -283,17 +283,30 @@ __global__ void k_gp(const float *__restrict__ opd, const float *__restrict__ gi
     }
 }
 
-// alpha_k = (r.z)_k / (p.Ap), reduced by the last block of the p.Ap producer.
-__device__ __forceinline__ void cg_alpha_last(const double *part_b, const CgScal &S, int b, int k) {
-    if (last_block(S.cnt + b, gridDim.x) && threadIdx.x < 32) {
-        const double pap = warp_sum_fresh(part_b, gridDim.x);
-        if (threadIdx.x == 0) {
-            double a = S.sc[(size_t)b * S.nsc + k] / pap;
-            if (!isfinite(a)) a = 0;  // pcg.c:80-83, pcg.cu:27-30
-            S.ab[2 * b] = (float)a;
-            S.cnt[b] = 0;
-        }
+// The p.Ap partials that the operator left, n per instance.  Whoever updates
+// x and r forms alpha from them: the producers need no fence, counter and last
+// block, whose three round trips came after everything else (k_hxt_rows, one 8
+// m LTAO instance 7.2 -> 5.3 us; k_spmv_lr, 32 30 m instances 32 -> 22 us).
+struct PapParts {
+    const double *part;  // [b][n]
+    int n;
+};
+// alpha_k = (r.z)_k / (p.Ap), by one warp; valid in every lane.
+__device__ __forceinline__ float cg_alpha(const PapParts &P, const CgScal &S, int b, int k) {
+    const double *part = P.part + (size_t)b * P.n;
+    const double rz = S.sc[(size_t)b * S.nsc + k];
+    double v = 0;
+    for (int i0 = threadIdx.x & 31; i0 < P.n; i0 += 4 * 32) {
+        double u[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) u[q] = i0 + 32 * q < P.n ? part[i0 + 32 * q] : 0.0;
+#pragma unroll
+        for (int q = 0; q < 4; q++) v += u[q];
     }
+    v = warp_sum(v);
+    double a = rz / __shfl_sync(0xffffffffu, v, 0);
+    if (!isfinite(a)) a = 0;  // pcg.c:80-83, pcg.cu:27-30
+    return (float)a;
 }
 
 struct LowRank {
@@ -308,8 +321,8 @@ struct LowRank {
 // fx[((w*ndm + l)*maxn + jx)*kx + e] and the y list (padding: weight 0).
 // Every load of a direction depends only on (w, jx, jy), so the loads of
 // several directions are in flight together.  Plus the low-rank NW term, an
-// optional vector added as is (the slaving term), and the p.Ap partials (last
-// block: alpha) for FitL.  grid: (ceil(nact/256), nb).
+// optional vector added as is (the slaving term), and the p.Ap partials for
+// FitL.  grid: (ceil(nact/256), nb).
 constexpr int kFitPad = 4;  // widest padded fit list
 struct FitPad {
     const GatherW *x, *y;
@@ -319,7 +332,7 @@ struct FitPad {
 __global__ void __launch_bounds__(kThreads)
 k_fit_hxt(const float *__restrict__ opd2, const float *__restrict__ xin, float *__restrict__ out,
           double *__restrict__ dot_part, FitPad fpd, const __grid_constant__ LayerTab dl, int ndm, int nfit,
-          int nfx, int nfy, long nact, LowRank lr, CgScal S, int k, const float *__restrict__ addv,
+          int nfx, int nfy, long nact, LowRank lr, const float *__restrict__ addv,
           const int *__restrict__ act) {
     pdl_enter();
     if (inactive(act, blockIdx.y)) return;
@@ -380,7 +393,6 @@ k_fit_hxt(const float *__restrict__ opd2, const float *__restrict__ xin, float *
     if (dot_part) {
         dotv = block_sum(dotv, sh);
         if (threadIdx.x == 0) dot_part[(size_t)b * gridDim.x + blockIdx.x] = dotv;
-        cg_alpha_last(dot_part + (size_t)b * gridDim.x, S, b, k);
     }
 }
 
@@ -649,7 +661,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_pupil_rows_group(const __grid_c
     pupil_rows_body<FROM_X, POS>(bid, a);
 }
 
-// Hx^T over all WFS, + L2^T L2 x and p.Ap partials (last block: alpha).  A
+// Hx^T over all WFS, + L2^T L2 x and p.Ap partials.  A
 // thread owns one layer column and RT consecutive layer rows.  For each WFS it
 // walks the pupil rows that reach them: the x half of the transpose (the
 // column's list: consecutive pupil columns, so K loads at one address) gives
@@ -676,7 +688,9 @@ struct HxtIndex {
     const float *yw;   // [(woff + (w*groups + g)*n + i) * RT + r]: weight of pupil row y0 + i to layer row g*RT + r
 };
 // Pupil rows whose loads go together: what RT rows of a layer sampled as the
-// pupil need (a layer at half the sampling takes two chunks).
+// pupil need (a layer at half the sampling takes two chunks).  With 5 for every
+// RT, windows of one or two rows were padded to it: one 30 m instance's step of
+// 10 iterations 459 -> 444 us.
 __host__ __device__ constexpr int hxt_chunk(int k, int rt) { return k > 4 ? 2 : rt == 4 ? 5 : rt == 2 ? 3 : 2; }
 // WFS whose loads go together: with one row per thread the launch is too small
 // to hide a WFS's two round trips behind other warps.
@@ -693,8 +707,6 @@ struct HxtArgs {
     int nps, nwfs, orows, ostride;  // rows of a WFS's plane of o, and their stride
     long nxtot;
     int do_l2;
-    CgScal S;
-    int kit;
     const int *act;
 };
 
@@ -844,17 +856,7 @@ __device__ __forceinline__ void hxt_rows_body(const uint3 bid, const unsigned gx
     }
     if (A.dot_part) {
         dotv = block_sum(dotv, sh);
-        double *part = A.dot_part + (size_t)b * gx;
-        if (threadIdx.x == 0) part[bid.x] = dotv;
-        if (last_block(A.S.cnt + b, gx) && threadIdx.x < 32) {  // alpha_k = (r.z)_k / (p.Ap)
-            const double pap = warp_sum_fresh(part, gx);
-            if (threadIdx.x == 0) {
-                double a = A.S.sc[(size_t)b * A.S.nsc + A.kit] / pap;
-                if (!isfinite(a)) a = 0;  // pcg.c:80-83, pcg.cu:27-30
-                A.S.ab[2 * b] = (float)a;
-                A.S.cnt[b] = 0;
-            }
-        }
+        if (threadIdx.x == 0) A.dot_part[(size_t)b * gx + bid.x] = dotv;
     }
 }
 
@@ -956,7 +958,7 @@ __device__ __forceinline__ void cg_rz_last(const double *part_b, const CgScal &S
             } else {
                 double be = rz / S.sc[(size_t)b * S.nsc + k];
                 if (!isfinite(be)) be = 0;
-                S.ab[2 * b + 1] = (float)be;
+                S.be[b] = (float)be;
                 S.sc[(size_t)b * S.nsc + k + 1] = rz;
             }
             S.cnt[b] = 0;
@@ -988,13 +990,13 @@ __global__ void k_dot_self(const float *__restrict__ v, double *__restrict__ par
 // r (no preconditioner), produces beta.
 __global__ void k_cg_update_xr(float *__restrict__ x, float *__restrict__ r,
                                const float *__restrict__ p, const float *__restrict__ Ap,
-                               double *__restrict__ rr_part, long n, CgScal S, int k, int iters,
+                               double *__restrict__ rr_part, long n, PapParts pap, CgScal S, int k, int iters,
                                int z_is_r, const int *__restrict__ act) {
     pdl_enter();
     if (inactive(act, blockIdx.y)) return;
     __shared__ double sh[32];
     const int b = blockIdx.y;
-    const float a = S.ab[2 * b];
+    const float a = cg_alpha(pap, S, b, k);
     const long j = (long)blockIdx.x * blockDim.x + threadIdx.x;
     double v = 0;
     if (j < n) {
@@ -1052,7 +1054,7 @@ __global__ void k_cg_update_p(float *__restrict__ p, const float *__restrict__ z
             }
     }
     if (inactive(act, b)) return;
-    const float be = init ? 0.f : S.ab[2 * b + 1];
+    const float be = init ? 0.f : S.be[b];
     float r[kUpdP];
 #pragma unroll
     for (int u = 0; u < kUpdP; u++) r[u] = init ? zv[u] : zv[u] + be * pv[u];
@@ -1098,8 +1100,15 @@ struct FdLayer {
     signed char rx[8], ry[8];
     int px, py;          // two-pass factor pair (index into kFftPairs) along x and y, -1: stages
 };
-struct FdTab {  // per layer, by value (kernel parameter space)
+// Layers of one size whose inverse transforms a CTA does together.
+struct FdGroup {
+    int n;
+    signed char l[kMaxLayers];
+};
+struct FdTab {  // per layer and group, by value (kernel parameter space)
     FdLayer l[kMaxLayers];
+    int ng;
+    FdGroup g[kMaxLayers];
 };
 
 // Lengths the two-pass FFT handles, as n = N1 * N2 (both passes' DFTs held
@@ -1353,9 +1362,9 @@ constexpr int kFusedThreads = 512;
 
 // Forward: r (instance-major) -> half spectra H.  grid: (nps, nb), block:
 // kFftThreads; dynamic shared memory: two buffers of `bufn` complex values,
-// then the layer's twiddle tables for n = nx and n = ny.  With `ab`, the CG
-// update of this iteration comes first on the layer's points:
-// x += alpha p, r -= alpha Ap (alpha = ab[2b]), and the updated r is
+// then the layer's twiddle tables for n = nx and n = ny.  With `xw`, the CG
+// update of iteration kit comes first on the layer's points:
+// x += alpha p, r -= alpha Ap, and the updated r is
 // transformed (the k_cg_update_xr of a non-final iteration, fused).  A thread
 // issues the loads of kFdLoads row pairs before using any of them, so the
 // global round trips overlap instead of following one another.
@@ -1364,7 +1373,7 @@ constexpr int kFdLoads = 5;
 __global__ void __launch_bounds__(kFftThreads, 2)
 k_fd_fwd(float *__restrict__ r, cplx *__restrict__ H, const __grid_constant__ FdTab ft, const cplx *__restrict__ tw,
          long nxtot, int bufn, float *__restrict__ xw, const float *__restrict__ pv,
-         const float *__restrict__ Apv, const float *__restrict__ ab, const int *__restrict__ act) {
+         const float *__restrict__ Apv, PapParts pap, CgScal SC, int kit, const int *__restrict__ act) {
     pdl_enter();
     if (inactive(act, blockIdx.y)) return;
     extern __shared__ cplx fsm[];
@@ -1374,12 +1383,12 @@ k_fd_fwd(float *__restrict__ r, cplx *__restrict__ H, const __grid_constant__ Fd
     cplx *A = fsm, *B = fsm + bufn, *twx = fsm + 2 * bufn, *twy = twx + nx;
     for (int i = threadIdx.x; i < nx; i += blockDim.x) twx[i] = tw[L.twx + i];
     for (int i = threadIdx.x; i < ny; i += blockDim.x) twy[i] = tw[L.twy + i];
+    const float a = xw ? cg_alpha(pap, SC, b, kit) : 0.f;  // every warp for itself: no barrier before the loads
     const size_t base = (size_t)b * nxtot + L.off;
     float *rb = r + base;
     const int xs = blockDim.x / nx, x0 = threadIdx.x / nx, xc = threadIdx.x - x0 * nx;  // nx <= blockDim
     if (x0 < xs) {
-        if (ab) {
-            const float a = ab[2 * b];
+        if (xw) {
             float *xb = xw + base;
             const float *pb = pv + base, *qb = Apv + base;
             for (int p0 = x0; p0 < np2; p0 += kFdLoads * xs) {
@@ -1766,7 +1775,8 @@ __device__ __forceinline__ double dsm_peer_f64(const double *local, unsigned ran
 // The vector part of an unpreconditioned CG iteration in one launch, a
 // thread-block cluster per instance: x += alpha p, r -= alpha Ap, r.r over the
 // cluster, beta, p = r + beta p, and (fit) t = V' p, what the next A p needs
-// of the low-rank term.  init: r = b - Ap (Ap = A x), b.b, r.r, p = r, t.  The
+// of the low-rank term (and p interleaved over il instances in pil, as its
+// sparse rows read it).  init: r = b - Ap (Ap = A x), b.b, r.r, p = r, t.  The
 // elements stay in registers between the passes.  The last iteration leaves
 // the residual instead of p.  Launch-bound: one launch of 4-9 us where the
 // update of x and r, the update of p and V' p took three of 3.7, 1.8 and 4-14
@@ -1777,13 +1787,13 @@ constexpr int kStepThreads = 512;
 template <int E>
 __global__ void __launch_bounds__(kStepThreads)
 k_cg_step(float *__restrict__ x, float *__restrict__ r, float *__restrict__ p, const float *__restrict__ Ap,
-          const float *__restrict__ bvec, long n, CgScal S, int k, int iters, int init, const float *__restrict__ V,
-          int nq, float *__restrict__ t, const int *__restrict__ act) {
+          const float *__restrict__ bvec, long n, PapParts pap, CgScal S, int k, int iters, int init,
+          const float *__restrict__ V, int nq, float *__restrict__ t, float *__restrict__ pil, int il, const int *__restrict__ act) {
     pdl_enter();
     if (inactive(act, blockIdx.y)) return;  // the whole cluster
     __shared__ double sh[kStepThreads / 32], sh2[kStepThreads / 32], s_part[2], s_lr[kMaxLr];
     __shared__ double s_w[kStepThreads / 32][kMaxLr];
-    __shared__ float s_beta;
+    __shared__ float s_beta, s_alpha;
     const int b = blockIdx.y, C = gridDim.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const size_t ob = (size_t)b * n;
     const long j0 = (long)blockIdx.x * (kStepThreads * E) + threadIdx.x;
@@ -1800,7 +1810,6 @@ k_cg_step(float *__restrict__ x, float *__restrict__ r, float *__restrict__ p, c
             rr += (double)rv[e] * rv[e];
         }
     } else {
-        const float a = S.ab[2 * b];
         float xv[E], av[E];
 #pragma unroll
         for (int e = 0; e < E; e++) {
@@ -1810,6 +1819,12 @@ k_cg_step(float *__restrict__ x, float *__restrict__ r, float *__restrict__ p, c
             xv[e] = j < n ? x[ob + j] : 0.f;
             av[e] = j < n ? Ap[ob + j] : 0.f;
         }
+        if (wid == 0) {
+            const float v = cg_alpha(pap, S, b, k);
+            if (lane == 0) s_alpha = v;
+        }
+        __syncthreads();
+        const float a = s_alpha;
 #pragma unroll
         for (int e = 0; e < E; e++) {
             const long j = j0 + e * kStepThreads;
@@ -1863,6 +1878,7 @@ k_cg_step(float *__restrict__ x, float *__restrict__ r, float *__restrict__ p, c
         if (j < n) {
             r[ob + j] = rv[e];
             if (!last) p[ob + j] = pv[e];
+            if (!last && pil) pil[((size_t)(b / il) * n + j) * il + b % il] = pv[e];
         }
     }
     if (nq && !last) {
@@ -1897,15 +1913,16 @@ k_cg_step(float *__restrict__ x, float *__restrict__ r, float *__restrict__ p, c
 }
 
 // Inverse: half spectra H -> z (instance-major), plus the r.z partial of this
-// (layer, instance); the last CTA of an instance leaves (r.z)_0 or beta.
-// grid: (nps, nb); shared memory as k_fd_fwd.
-// PU (CG step, launched as clusters of the nps layer CTAs of one instance):
+// (group, instance); the last CTA of an instance leaves (r.z)_0 or beta.
+// grid: (groups, nb); shared memory as k_fd_fwd.
+// GRP: some group has more than one layer.
+// PU (CG step, launched as clusters of the group CTAs of one instance):
 // the CTAs exchange their r.z partials through distributed shared memory
 // behind a cluster barrier, each forms r.z (same order, same value) and
 // beta, and updates its own layer of p = z + beta p (init: p = z), which
 // replaces the separate p update launch; z is not written.  Rank 0 records
 // the CG scalars as cg_rz_last does.
-template <bool PU>
+template <bool PU, bool GRP>
 __global__ void __launch_bounds__(kFftThreads, 2)
 k_fd_inv(const cplx *__restrict__ H, const float *__restrict__ r, float *__restrict__ z,
          double *__restrict__ rz_part, const __grid_constant__ FdTab ft, const cplx *__restrict__ tw, long nxtot,
@@ -1914,36 +1931,45 @@ k_fd_inv(const cplx *__restrict__ H, const float *__restrict__ r, float *__restr
     if (inactive(act, blockIdx.y)) return;
     extern __shared__ cplx fsm[];
     __shared__ double sh[32];
-    const FdLayer &L = ft.l[blockIdx.x];
+    const FdGroup &G = ft.g[blockIdx.x];
+    const FdLayer &L = ft.l[G.l[0]];  // the size and tables of all of them
     const int b = blockIdx.y;
     const int nx = L.nx, ny = L.ny, h = nx / 2 + 1, np2 = ny / 2;
+    const int nr = GRP ? G.n * np2 : np2, nc = GRP ? G.n * h : h;  // row pairs and half-spectrum columns of the group
     cplx *A = fsm, *B = fsm + bufn, *twx = fsm + 2 * bufn, *twy = twx + nx;
     for (int i = threadIdx.x; i < nx; i += blockDim.x) twx[i] = tw[L.twx + i];
     for (int i = threadIdx.x; i < ny; i += blockDim.x) twy[i] = tw[L.twy + i];
-    const cplx *in = H + L.hoff + (size_t)b * L.hs;
     constexpr int kLd = 2 * kFdLoads;  // spectrum values a thread loads before storing any
-    for (int i0 = threadIdx.x; i0 < ny * h; i0 += kLd * blockDim.x) {
-        cplx v[kLd];
+    {
+        const int cs = blockDim.x / nc, q0 = threadIdx.x / nc, c = threadIdx.x - q0 * nc, g = GRP ? c / h : 0;  // nc <= blockDim
+        if (q0 < cs) {
+            const FdLayer &F = GRP ? ft.l[G.l[g]] : L;
+            const cplx *in = H + F.hoff + (size_t)b * F.hs + (c - g * h);
+            for (int i0 = q0; i0 < ny; i0 += kLd * cs) {
+                cplx v[kLd];
 #pragma unroll
-        for (int u = 0; u < kLd; u++) {
-            const int i = i0 + u * blockDim.x;
-            if (i < ny * h) v[u] = in[i];
-        }
+                for (int u = 0; u < kLd; u++) {
+                    const int i = i0 + u * cs;
+                    if (i < ny) v[u] = in[i * h];
+                }
 #pragma unroll
-        for (int u = 0; u < kLd; u++) {
-            const int i = i0 + u * blockDim.x;
-            if (i < ny * h) A[i] = v[u];
+                for (int u = 0; u < kLd; u++) {
+                    const int i = i0 + u * cs;
+                    if (i < ny) A[i * nc + c] = v[u];
+                }
+            }
         }
     }
     __syncthreads();
-    cplx *C = fft_dir<false>(L.py, A, B, ny, h, h, L.ry, L.nry, twy, true);
+    cplx *C = fft_dir<false>(L.py, A, B, ny, nc, nc, L.ry, L.nry, twy, true);
     cplx *Zb = (C == A) ? B : A;
     const int xs = blockDim.x / nx, x0 = threadIdx.x / nx, k = threadIdx.x - x0 * nx;
-    for (int p = x0; x0 < xs && p < np2; p += xs) {
-        const int i = p * nx + k;
+    for (int p = x0; x0 < xs && p < nr; p += xs) {
+        const int i = p * nx + k, g = GRP ? p / np2 : 0;
         const bool hi = k > nx / 2;
         const int kk = hi ? nx - k : k;
-        cplx a = C[(2 * p) * h + kk], c = C[(2 * p + 1) * h + kk];
+        const cplx *s = C + 2 * (p - g * np2) * nc + g * h + kk;
+        cplx a = s[0], c = s[nc];
         if (kk == 0 || kk == nx / 2) {
             a.y = 0.f;
             c.y = 0.f;
@@ -1955,29 +1981,36 @@ k_fd_inv(const cplx *__restrict__ H, const float *__restrict__ r, float *__restr
         Zb[i] = make_float2(a.x - c.y, a.y + c.x);  // a + i c
     }
     __syncthreads();
-    const cplx *Zo = fft_dir<true>(L.px, Zb, C, nx, np2, nx, L.rx, L.nrx, twx, true);
-    const size_t base = (size_t)b * nxtot + L.off;
+    const cplx *Zo = fft_dir<true>(L.px, Zb, C, nx, nr, nx, L.rx, L.nrx, twx, true);
+    const size_t base = (size_t)b * nxtot;
+    const float *rb = r + base;
+    float *zb = z + base, *pb = pv + base;  // one of them is written
+    // first point of row pair p of the group
+    auto pair_at = [&](int p) {
+        const int g = GRP ? p / np2 : 0;
+        return (int)(GRP ? ft.l[G.l[g]].off : L.off) + 2 * (p - g * np2) * nx + k;
+    };
     double v = 0;
-    for (int p0 = x0; x0 < xs && p0 < np2; p0 += kFdLoads * xs) {
+    for (int p0 = x0; x0 < xs && p0 < nr; p0 += kFdLoads * xs) {
         float rv[kFdLoads][2];
+        int at[kFdLoads];
 #pragma unroll
         for (int u = 0; u < kFdLoads; u++) {
             const int p = p0 + u * xs;
-            if (p < np2) {
-                const size_t o0 = base + (size_t)(2 * p) * nx + k;
-                rv[u][0] = r[o0];
-                rv[u][1] = r[o0 + nx];
+            if (p < nr) {
+                at[u] = pair_at(p);
+                rv[u][0] = rb[at[u]];
+                rv[u][1] = rb[at[u] + nx];
             }
         }
 #pragma unroll
         for (int u = 0; u < kFdLoads; u++) {
             const int p = p0 + u * xs;
-            if (p < np2) {
+            if (p < nr) {
                 const cplx q = Zo[p * nx + k];
-                const size_t o0 = base + (size_t)(2 * p) * nx + k, o1 = o0 + nx;
                 if (!PU) {
-                    z[o0] = q.x;
-                    z[o1] = q.y;
+                    zb[at[u]] = q.x;
+                    zb[at[u] + nx] = q.y;
                 }
                 v += (double)q.x * rv[u][0] + (double)q.y * rv[u][1];
             }
@@ -2013,7 +2046,7 @@ k_fd_inv(const cplx *__restrict__ H, const float *__restrict__ r, float *__restr
                     if (init) {  // start (or restart) at iteration kit
                         SC.sc[(size_t)b * SC.nsc + kit] = rz;
                     } else {
-                        SC.ab[2 * b + 1] = (float)be;
+                        SC.be[b] = (float)be;
                         SC.sc[(size_t)b * SC.nsc + kit + 1] = rz;
                     }
                 }
@@ -2022,25 +2055,27 @@ k_fd_inv(const cplx *__restrict__ H, const float *__restrict__ r, float *__restr
         __syncthreads();
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // done reading the others
         const float be = (float)s_be;
-        for (int p0 = x0; x0 < xs && p0 < np2; p0 += kFdLoads * xs) {
+        for (int p0 = x0; x0 < xs && p0 < nr; p0 += kFdLoads * xs) {
             float pp[kFdLoads][2];
+            int at[kFdLoads];
 #pragma unroll
             for (int u = 0; u < kFdLoads; u++) {
                 const int p = p0 + u * xs;
-                if (p < np2 && !init) {
-                    const size_t o0 = base + (size_t)(2 * p) * nx + k;
-                    pp[u][0] = pv[o0];
-                    pp[u][1] = pv[o0 + nx];
+                if (p < nr) {
+                    at[u] = pair_at(p);
+                    if (!init) {
+                        pp[u][0] = pb[at[u]];
+                        pp[u][1] = pb[at[u] + nx];
+                    }
                 }
             }
 #pragma unroll
             for (int u = 0; u < kFdLoads; u++) {
                 const int p = p0 + u * xs;
-                if (p < np2) {
+                if (p < nr) {
                     const cplx q = Zo[p * nx + k];
-                    const size_t o0 = base + (size_t)(2 * p) * nx + k;
-                    pv[o0] = init ? q.x : q.x + be * pp[u][0];
-                    pv[o0 + nx] = init ? q.y : q.y + be * pp[u][1];
+                    pb[at[u]] = init ? q.x : q.x + be * pp[u][0];
+                    pb[at[u] + nx] = init ? q.y : q.y + be * pp[u][1];
                 }
             }
         }
@@ -2128,7 +2163,7 @@ __device__ void fft_dir_inplace(int pair, cplx *a, cplx *b, int n, int count, in
 __global__ void __launch_bounds__(kFusedThreads, 1)
 k_fd_fused(float *__restrict__ r, const __grid_constant__ FdTab ft, const __grid_constant__ FdFusedTab fu,
            const cplx *__restrict__ tw, const cplx *__restrict__ M, const FdMem *__restrict__ mem, int bs,
-           long nxtot, float *__restrict__ xw, const float *__restrict__ Apv, CgScal SC, int kit, int init,
+           long nxtot, float *__restrict__ xw, const float *__restrict__ Apv, PapParts pap, CgScal SC, int kit, int init,
            const int *__restrict__ act, float *__restrict__ pv) {
     pdl_enter();
     // an instance's CTAs are one cluster: all return or none does
@@ -2152,8 +2187,8 @@ k_fd_fused(float *__restrict__ r, const __grid_constant__ FdTab ft, const __grid
     // registers for the r.z and the p update at the end.
     const bool one = npr <= kFdLoads * xs;
     float rv[kFdLoads][2], pp[kFdLoads][2];
+    const float a = xw ? cg_alpha(pap, SC, b, kit) : 0.f;  // every warp for itself
     if (x0 < xs) {
-        const float a = SC.ab ? SC.ab[2 * b] : 0.f;
         for (int p0 = P.p0 + x0; p0 < P.p1; p0 += kFdLoads * xs) {
             float xv[kFdLoads][2], qq[kFdLoads][2];
 #pragma unroll
@@ -2323,7 +2358,7 @@ k_fd_fused(float *__restrict__ r, const __grid_constant__ FdTab ft, const __grid
                 if (init) {  // start (or restart) at iteration kit
                     SC.sc[(size_t)b * SC.nsc + kit] = t;
                 } else {
-                    SC.ab[2 * b + 1] = (float)be;
+                    SC.be[b] = (float)be;
                     SC.sc[(size_t)b * SC.nsc + kit + 1] = t;
                 }
             }
