@@ -314,6 +314,9 @@ struct Recon {
                   const float *Apupd = nullptr, float *pnext = nullptr);
     using FdInvKern = void (*)(const cplx *, const float *, float *, double *, FdTab, const cplx *, long, int, CgScal, int,
                                int, const int *, float *);
+    using FdFwdKern = void (*)(float *, cplx *, FdTab, const cplx *, long, int, float *, const float *, const float *, PapParts,
+                               CgScal, int, const int *);
+    FdFwdKern fd_fwd_kern() const { return fdtab.ng < nps ? k_fd_fwd<true> : k_fd_fwd<false>; }
     FdInvKern fd_inv_kern(bool pu) const {  // by whether its groups hold several layers
         return fdtab.ng < nps ? (pu ? k_fd_inv<true, true> : k_fd_inv<false, true>)
                               : (pu ? k_fd_inv<true, false> : k_fd_inv<false, false>);
@@ -1044,13 +1047,15 @@ void Recon::build_fdpcg(const mb_fdpcg_desc *fd) {
         }
         twn = std::max(twn, F.nx + F.ny);
     }
-    // The inverse's groups: equal layers together, up to the points (and a CTA's
-    // columns) of the largest layer, once an instance's CTAs no longer run all
-    // at once.  Its cluster then holds CTAs of equal work: with one layer each,
-    // the small layers' CTAs kept their places on the SMs until the largest's
-    // were done (30 m, 256 instances: 91 -> 70 us).  While all CTAs are resident
-    // a group only lengthens the chain (6 instances: 12.4 -> 16 us).  Each layer
-    // alone, too, where the groups' buffers would leave fewer CTAs on an SM.
+    // Groups: equal layers together, up to the points (and a CTA's columns) of
+    // the largest layer, once there are more layers to transform than SMs.  An
+    // instance's CTAs then have equal work; with a layer each, the small layers'
+    // CTAs of the inverse's cluster kept their places on the SMs until the
+    // largest's were done.  30 m, forward and inverse: 32 instances 16.2 + 17.8
+    // -> 12.4 + 15.6 us, 256 instances 66.7 + 95.7 -> 58.2 + 63.8.  With SMs to
+    // spare a group only lengthens the chain (8 instances: 11.0 + 13.2 against
+    // 12.0 + 15.0).  Each layer alone, too, where the groups' buffers would leave
+    // fewer CTAs on an SM.
     auto buffers = [&](long limit) {
         fdtab.ng = fd_bufn = 0;
         for (int l = 0; l < nps; l++) {
@@ -1059,10 +1064,13 @@ void Recon::build_fdpcg(const mb_fdpcg_desc *fd) {
             for (; g < fdtab.ng; g++) {
                 const FdGroup &Q = fdtab.g[g];
                 if (fl[Q.l[0]].nx == F.nx && fl[Q.l[0]].ny == F.ny && (Q.n + 1L) * F.nx * F.ny <= limit &&
-                    (Q.n + 1) * (F.nx / 2 + 1) <= kFftThreads)
+                    (Q.n + 1) * (F.nx / 2 + 1) <= kFftThreads && (Q.n + 1L) * (F.ny / 2) * (F.ny / 2) < 65536)
                     break;
             }
-            if (g == fdtab.ng) fdtab.g[fdtab.ng++] = FdGroup{};
+            if (g == fdtab.ng) {
+                fdtab.g[fdtab.ng++] = FdGroup{};
+                fdtab.g[g].inv_np2 = (65536 + F.ny / 2 - 1) / (F.ny / 2);
+            }
             fdtab.g[g].l[fdtab.g[g].n++] = (signed char)l;
         }
         for (int g = 0; g < fdtab.ng; g++) {
@@ -1078,14 +1086,14 @@ void Recon::build_fdpcg(const mb_fdpcg_desc *fd) {
     for (const FdLayer &F : fl) most = std::max(most, (long)F.nx * F.ny);
     constexpr size_t kSmSmem = 227 * 1024, kPerCta = 1024;
     const size_t alone = buffers(0);
-    fd_smem = (long)nb * nps > 2 * 148 ? buffers(most) : alone;
+    fd_smem = (long)nb * nps > 148 ? buffers(most) : alone;
     if (fd_smem > 200 * 1024 || kSmSmem / (fd_smem + kPerCta) < std::min<size_t>(2, kSmSmem / (alone + kPerCta)))
         fd_smem = buffers(0);
     fd_lay.upload(fl);
     for (int l = 0; l < nps; l++) fdtab.l[l] = fl[l];
     fd_tw.upload(tw);
     MB_REQUIRE(fd_smem <= 200 * 1024, "fdpcg: layer FFT needs %zu bytes of shared memory", fd_smem);
-    MB_CUDA_TRY(cudaFuncSetAttribute(k_fd_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fd_smem));
+    MB_CUDA_TRY(cudaFuncSetAttribute(fd_fwd_kern(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fd_smem));
     for (bool pu : {false, true})
         MB_CUDA_TRY(cudaFuncSetAttribute(fd_inv_kern(pu), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fd_smem));
     // the CG step's inverse runs as clusters of the group CTAs of an instance when such a cluster fits
@@ -1514,7 +1522,7 @@ bool Recon::op_fdpcg(float *rin, float *zout, double *rzp, cudaStream_t s, int k
                        PapParts{pap_part.p, nblk_hxt}, scal(), k, init, act(), pnext);
         return true;
     }
-    launch(k_fd_fwd, dim3(nps, nb), dim3(kFftThreads), fd_smem, s, rin, spec.p, fdtab, fd_tw.p, nxtot, fd_bufn, xupd,
+    launch(fd_fwd_kern(), dim3(fdtab.ng, nb), dim3(kFftThreads), fd_smem, s, rin, spec.p, fdtab, fd_tw.p, nxtot, fd_bufn, xupd,
            pupd, Apupd, PapParts{pap_part.p, nblk_hxt}, scal(), k, act());
     fd_mul(s);
     CgScal S = in_cg ? scal() : CgScal{};
@@ -1996,7 +2004,7 @@ void Recon::time_stages(int reps, float *ms, double *bytes, int *launches) {
                            stream, rhs.p, z.p, nxtot, scal(), 0, act());
                     break;
                 case 4:
-                    launch(k_fd_fwd, dim3(nps, nb), dim3(kFftThreads), fd_smem, stream, rhs.p, spec.p, fdtab,
+                    launch(fd_fwd_kern(), dim3(fdtab.ng, nb), dim3(kFftThreads), fd_smem, stream, rhs.p, spec.p, fdtab,
                            fd_tw.p, nxtot, fd_bufn, z.p, p.p, Ap.p, PapParts{pap_part.p, nblk_hxt}, scal(), 0, act());
                     break;
                 case 5: fd_mul(stream); break;

@@ -1100,9 +1100,10 @@ struct FdLayer {
     signed char rx[8], ry[8];
     int px, py;          // two-pass factor pair (index into kFftPairs) along x and y, -1: stages
 };
-// Layers of one size whose inverse transforms a CTA does together.
+// Layers of one size whose transforms a CTA does together.
 struct FdGroup {
     int n;
+    int inv_np2;  // ceil(2^16 / row pairs of a layer): p / np2 = p * inv_np2 >> 16 for the group's row pairs
     signed char l[kMaxLayers];
 };
 struct FdTab {  // per layer and group, by value (kernel parameter space)
@@ -1360,8 +1361,8 @@ constexpr int kFftThreads = 512;  // threads of a layer-FFT CTA
 // 512, 1.16-1.17 with 256, 1.37 with 1024, which spills)
 constexpr int kFusedThreads = 512;
 
-// Forward: r (instance-major) -> half spectra H.  grid: (nps, nb), block:
-// kFftThreads; dynamic shared memory: two buffers of `bufn` complex values,
+// Forward: r (instance-major) -> half spectra H.  grid: (groups, nb), block:
+// kFftThreads (GRP: some group has more than one layer); dynamic shared memory: two buffers of `bufn` complex values,
 // then the layer's twiddle tables for n = nx and n = ny.  With `xw`, the CG
 // update of iteration kit comes first on the layer's points:
 // x += alpha p, r -= alpha Ap, and the updated r is
@@ -1370,6 +1371,7 @@ constexpr int kFusedThreads = 512;
 // global round trips overlap instead of following one another.
 constexpr int kFdLoads = 5;
 
+template <bool GRP>
 __global__ void __launch_bounds__(kFftThreads, 2)
 k_fd_fwd(float *__restrict__ r, cplx *__restrict__ H, const __grid_constant__ FdTab ft, const cplx *__restrict__ tw,
          long nxtot, int bufn, float *__restrict__ xw, const float *__restrict__ pv,
@@ -1377,84 +1379,111 @@ k_fd_fwd(float *__restrict__ r, cplx *__restrict__ H, const __grid_constant__ Fd
     pdl_enter();
     if (inactive(act, blockIdx.y)) return;
     extern __shared__ cplx fsm[];
-    const FdLayer &L = ft.l[blockIdx.x];
+    __shared__ float s_a;
+    const FdGroup &G = ft.g[blockIdx.x];
+    const FdLayer &L = ft.l[G.l[0]];  // the size and tables of all of them
     const int b = blockIdx.y;
     const int nx = L.nx, ny = L.ny, h = nx / 2 + 1, np2 = ny / 2;
+    const int nr = GRP ? G.n * np2 : np2, nc = GRP ? G.n * h : h;  // row pairs and half-spectrum columns
     cplx *A = fsm, *B = fsm + bufn, *twx = fsm + 2 * bufn, *twy = twx + nx;
     for (int i = threadIdx.x; i < nx; i += blockDim.x) twx[i] = tw[L.twx + i];
     for (int i = threadIdx.x; i < ny; i += blockDim.x) twy[i] = tw[L.twy + i];
-    const float a = xw ? cg_alpha(pap, SC, b, kit) : 0.f;  // every warp for itself: no barrier before the loads
-    const size_t base = (size_t)b * nxtot + L.off;
-    float *rb = r + base;
+    const size_t base = (size_t)b * nxtot;
+    float *rb = r + base, *xb = xw + base;
+    const float *pb = pv + base, *qb = Apv + base;
     const int xs = blockDim.x / nx, x0 = threadIdx.x / nx, xc = threadIdx.x - x0 * nx;  // nx <= blockDim
-    if (x0 < xs) {
-        if (xw) {
-            float *xb = xw + base;
-            const float *pb = pv + base, *qb = Apv + base;
-            for (int p0 = x0; p0 < np2; p0 += kFdLoads * xs) {
-                float xv[kFdLoads][2], pp[kFdLoads][2], rv[kFdLoads][2], qq[kFdLoads][2];
+    // first point of row pair p, in an instance vector
+    auto pair_at = [&](int p) {
+        const int g = GRP ? p * G.inv_np2 >> 16 : 0;
+        return (int)(GRP ? ft.l[G.l[g]].off : L.off) + 2 * (p - g * np2) * nx + xc;
+    };
+    const int end = x0 < xs ? nr : 0;  // threads past the last whole row load nothing
+    if (xw) {
+        float a = 0.f;
+        for (int q0 = 0; q0 < nr; q0 += kFdLoads * xs) {
+            const int p0 = q0 + x0;
+            float xv[kFdLoads][2], pp[kFdLoads][2], rv[kFdLoads][2], qq[kFdLoads][2];
 #pragma unroll
-                for (int u = 0; u < kFdLoads; u++) {
-                    const int p = p0 + u * xs;
-                    if (p < np2) {
-                        const int o0 = (2 * p) * nx + xc, o1 = o0 + nx;
-                        xv[u][0] = xb[o0];
-                        xv[u][1] = xb[o1];
-                        pp[u][0] = pb[o0];
-                        pp[u][1] = pb[o1];
-                        rv[u][0] = rb[o0];
-                        rv[u][1] = rb[o1];
-                        qq[u][0] = qb[o0];
-                        qq[u][1] = qb[o1];
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < kFdLoads; u++) {
-                    const int p = p0 + u * xs;
-                    if (p < np2) {
-                        const int o0 = (2 * p) * nx + xc, o1 = o0 + nx;
-                        xb[o0] = xv[u][0] + a * pp[u][0];
-                        xb[o1] = xv[u][1] + a * pp[u][1];
-                        const float r0 = rv[u][0] - a * qq[u][0], r1 = rv[u][1] - a * qq[u][1];
-                        rb[o0] = r0;
-                        rb[o1] = r1;
-                        A[p * nx + xc] = make_float2(r0, r1);
-                    }
+            for (int u = 0; u < kFdLoads; u++) {
+                const int p = p0 + u * xs;
+                if (p < end) {
+                    const int o0 = pair_at(p), o1 = o0 + nx;
+                    xv[u][0] = xb[o0];
+                    xv[u][1] = xb[o1];
+                    pp[u][0] = pb[o0];
+                    pp[u][1] = pb[o1];
+                    rv[u][0] = rb[o0];
+                    rv[u][1] = rb[o1];
+                    qq[u][0] = qb[o0];
+                    qq[u][1] = qb[o1];
                 }
             }
-        } else {
-            for (int p0 = x0; p0 < np2; p0 += kFdLoads * xs) {
-                float rv[kFdLoads][2];
-#pragma unroll
-                for (int u = 0; u < kFdLoads; u++) {
-                    const int p = p0 + u * xs;
-                    if (p < np2) {
-                        rv[u][0] = rb[(2 * p) * nx + xc];
-                        rv[u][1] = rb[(2 * p + 1) * nx + xc];
-                    }
+            if (q0 == 0) {  // alpha, while the first loads are on their way
+                if (threadIdx.x < 32) {
+                    const float v = cg_alpha(pap, SC, b, kit);
+                    if (threadIdx.x == 0) s_a = v;
                 }
+                __syncthreads();
+                a = s_a;
+            }
 #pragma unroll
-                for (int u = 0; u < kFdLoads; u++) {
-                    const int p = p0 + u * xs;
-                    if (p < np2) A[p * nx + xc] = make_float2(rv[u][0], rv[u][1]);
+            for (int u = 0; u < kFdLoads; u++) {
+                const int p = p0 + u * xs;
+                if (p < end) {
+                    const int o0 = pair_at(p), o1 = o0 + nx;
+                    xb[o0] = xv[u][0] + a * pp[u][0];
+                    xb[o1] = xv[u][1] + a * pp[u][1];
+                    const float r0 = rv[u][0] - a * qq[u][0], r1 = rv[u][1] - a * qq[u][1];
+                    rb[o0] = r0;
+                    rb[o1] = r1;
+                    A[p * nx + xc] = make_float2(r0, r1);
                 }
+            }
+        }
+    } else {
+        for (int p0 = x0; p0 < end; p0 += kFdLoads * xs) {
+            float rv[kFdLoads][2];
+#pragma unroll
+            for (int u = 0; u < kFdLoads; u++) {
+                const int p = p0 + u * xs;
+                if (p < end) {
+                    const int o0 = pair_at(p);
+                    rv[u][0] = rb[o0];
+                    rv[u][1] = rb[o0 + nx];
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < kFdLoads; u++) {
+                const int p = p0 + u * xs;
+                if (p < end) A[p * nx + xc] = make_float2(rv[u][0], rv[u][1]);
             }
         }
     }
     __syncthreads();
-    cplx *Z = fft_dir<true>(L.px, A, B, nx, np2, nx, L.rx, L.nrx, twx, false);
+    cplx *Z = fft_dir<true>(L.px, A, B, nx, nr, nx, L.rx, L.nrx, twx, false);
     cplx *S = (Z == A) ? B : A;
     const int hs_ = blockDim.x / h, h0 = threadIdx.x / h, k = threadIdx.x - h0 * h;
-    for (int p = h0; h0 < hs_ && p < np2; p += hs_) {
+    for (int p = h0; h0 < hs_ && p < nr; p += hs_) {
         const cplx zk = Z[p * nx + k], zm = cconj(Z[p * nx + (k == 0 ? 0 : nx - k)]);
-        S[(2 * p) * h + k] = make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y + zm.y));
+        const int g = GRP ? p * G.inv_np2 >> 16 : 0;
+        cplx *s = S + 2 * (p - g * np2) * nc + g * h + k;  // [ky][the group's columns]
+        s[0] = make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y + zm.y));
         const cplx d = csub(zk, zm);
-        S[(2 * p + 1) * h + k] = make_float2(0.5f * d.y, -0.5f * d.x);  // -i/2 (zk - conj(z_-k))
+        s[nc] = make_float2(0.5f * d.y, -0.5f * d.x);  // -i/2 (zk - conj(z_-k))
     }
     __syncthreads();
-    const cplx *C = fft_dir<false>(L.py, S, Z, ny, h, h, L.ry, L.nry, twy, false);
-    cplx *out = H + L.hoff + (size_t)b * L.hs;
-    for (int i = threadIdx.x; i < ny * h; i += blockDim.x) out[i] = C[i];
+    const cplx *C = fft_dir<false>(L.py, S, Z, ny, nc, nc, L.ry, L.nry, twy, false);
+    if constexpr (GRP) {
+        const int cs = blockDim.x / nc, q0 = threadIdx.x / nc, c = threadIdx.x - q0 * nc, g = c / h;  // nc <= blockDim
+        if (q0 < cs) {
+            const FdLayer &F = ft.l[G.l[g]];
+            cplx *out = H + F.hoff + (size_t)b * F.hs + (c - g * h);
+            for (int i = q0; i < ny; i += cs) out[i * h] = C[i * nc + c];
+        }
+    } else {
+        cplx *out = H + L.hoff + (size_t)b * L.hs;
+        for (int i = threadIdx.x; i < ny * h; i += blockDim.x) out[i] = C[i];
+    }
 }
 
 // Per-frequency block solve on the blocks of the non-positive x frequencies
@@ -1940,10 +1969,10 @@ k_fd_inv(const cplx *__restrict__ H, const float *__restrict__ r, float *__restr
     for (int i = threadIdx.x; i < nx; i += blockDim.x) twx[i] = tw[L.twx + i];
     for (int i = threadIdx.x; i < ny; i += blockDim.x) twy[i] = tw[L.twy + i];
     constexpr int kLd = 2 * kFdLoads;  // spectrum values a thread loads before storing any
-    {
-        const int cs = blockDim.x / nc, q0 = threadIdx.x / nc, c = threadIdx.x - q0 * nc, g = GRP ? c / h : 0;  // nc <= blockDim
+    if constexpr (GRP) {
+        const int cs = blockDim.x / nc, q0 = threadIdx.x / nc, c = threadIdx.x - q0 * nc, g = c / h;  // nc <= blockDim
         if (q0 < cs) {
-            const FdLayer &F = GRP ? ft.l[G.l[g]] : L;
+            const FdLayer &F = ft.l[G.l[g]];
             const cplx *in = H + F.hoff + (size_t)b * F.hs + (c - g * h);
             for (int i0 = q0; i0 < ny; i0 += kLd * cs) {
                 cplx v[kLd];
@@ -1959,13 +1988,28 @@ k_fd_inv(const cplx *__restrict__ H, const float *__restrict__ r, float *__restr
                 }
             }
         }
+    } else {
+        const cplx *in = H + L.hoff + (size_t)b * L.hs;
+        for (int i0 = threadIdx.x; i0 < ny * h; i0 += kLd * blockDim.x) {
+            cplx v[kLd];
+#pragma unroll
+            for (int u = 0; u < kLd; u++) {
+                const int i = i0 + u * blockDim.x;
+                if (i < ny * h) v[u] = in[i];
+            }
+#pragma unroll
+            for (int u = 0; u < kLd; u++) {
+                const int i = i0 + u * blockDim.x;
+                if (i < ny * h) A[i] = v[u];
+            }
+        }
     }
     __syncthreads();
     cplx *C = fft_dir<false>(L.py, A, B, ny, nc, nc, L.ry, L.nry, twy, true);
     cplx *Zb = (C == A) ? B : A;
     const int xs = blockDim.x / nx, x0 = threadIdx.x / nx, k = threadIdx.x - x0 * nx;
     for (int p = x0; x0 < xs && p < nr; p += xs) {
-        const int i = p * nx + k, g = GRP ? p / np2 : 0;
+        const int i = p * nx + k, g = GRP ? p * G.inv_np2 >> 16 : 0;
         const bool hi = k > nx / 2;
         const int kk = hi ? nx - k : k;
         const cplx *s = C + 2 * (p - g * np2) * nc + g * h + kk;
@@ -1987,20 +2031,19 @@ k_fd_inv(const cplx *__restrict__ H, const float *__restrict__ r, float *__restr
     float *zb = z + base, *pb = pv + base;  // one of them is written
     // first point of row pair p of the group
     auto pair_at = [&](int p) {
-        const int g = GRP ? p / np2 : 0;
+        const int g = GRP ? p * G.inv_np2 >> 16 : 0;
         return (int)(GRP ? ft.l[G.l[g]].off : L.off) + 2 * (p - g * np2) * nx + k;
     };
     double v = 0;
     for (int p0 = x0; x0 < xs && p0 < nr; p0 += kFdLoads * xs) {
         float rv[kFdLoads][2];
-        int at[kFdLoads];
 #pragma unroll
         for (int u = 0; u < kFdLoads; u++) {
             const int p = p0 + u * xs;
             if (p < nr) {
-                at[u] = pair_at(p);
-                rv[u][0] = rb[at[u]];
-                rv[u][1] = rb[at[u] + nx];
+                const int at = pair_at(p);
+                rv[u][0] = rb[at];
+                rv[u][1] = rb[at + nx];
             }
         }
 #pragma unroll
@@ -2009,8 +2052,9 @@ k_fd_inv(const cplx *__restrict__ H, const float *__restrict__ r, float *__restr
             if (p < nr) {
                 const cplx q = Zo[p * nx + k];
                 if (!PU) {
-                    zb[at[u]] = q.x;
-                    zb[at[u] + nx] = q.y;
+                    const int at = pair_at(p);
+                    zb[at] = q.x;
+                    zb[at + nx] = q.y;
                 }
                 v += (double)q.x * rv[u][0] + (double)q.y * rv[u][1];
             }
@@ -2057,16 +2101,13 @@ k_fd_inv(const cplx *__restrict__ H, const float *__restrict__ r, float *__restr
         const float be = (float)s_be;
         for (int p0 = x0; x0 < xs && p0 < nr; p0 += kFdLoads * xs) {
             float pp[kFdLoads][2];
-            int at[kFdLoads];
 #pragma unroll
             for (int u = 0; u < kFdLoads; u++) {
                 const int p = p0 + u * xs;
-                if (p < nr) {
-                    at[u] = pair_at(p);
-                    if (!init) {
-                        pp[u][0] = pb[at[u]];
-                        pp[u][1] = pb[at[u] + nx];
-                    }
+                if (p < nr && !init) {
+                    const int at = pair_at(p);
+                    pp[u][0] = pb[at];
+                    pp[u][1] = pb[at + nx];
                 }
             }
 #pragma unroll
@@ -2074,8 +2115,9 @@ k_fd_inv(const cplx *__restrict__ H, const float *__restrict__ r, float *__restr
                 const int p = p0 + u * xs;
                 if (p < nr) {
                     const cplx q = Zo[p * nx + k];
-                    pb[at[u]] = init ? q.x : q.x + be * pp[u][0];
-                    pb[at[u] + nx] = init ? q.y : q.y + be * pp[u][1];
+                    const int at = pair_at(p);
+                    pb[at] = init ? q.x : q.x + be * pp[u][0];
+                    pb[at + nx] = init ? q.y : q.y + be * pp[u][1];
                 }
             }
         }
@@ -2187,45 +2229,54 @@ k_fd_fused(float *__restrict__ r, const __grid_constant__ FdTab ft, const __grid
     // registers for the r.z and the p update at the end.
     const bool one = npr <= kFdLoads * xs;
     float rv[kFdLoads][2], pp[kFdLoads][2];
-    const float a = xw ? cg_alpha(pap, SC, b, kit) : 0.f;  // every warp for itself
-    if (x0 < xs) {
-        for (int p0 = P.p0 + x0; p0 < P.p1; p0 += kFdLoads * xs) {
-            float xv[kFdLoads][2], qq[kFdLoads][2];
+    __shared__ float s_a;
+    const int end = x0 < xs ? P.p1 : 0;  // threads past the last whole row load nothing
+    float a = 0.f;
+    for (int q0 = P.p0; q0 < P.p1; q0 += kFdLoads * xs) {
+        const int p0 = q0 + x0;
+        float xv[kFdLoads][2], qq[kFdLoads][2];
 #pragma unroll
-            for (int u = 0; u < kFdLoads; u++) {
-                const int p = p0 + u * xs;
-                if (p < P.p1) {
-                    const int o0 = (2 * p) * nx + xc, o1 = o0 + nx;
-                    rv[u][0] = rb[o0];
-                    rv[u][1] = rb[o1];
-                    if (xw) {
-                        xv[u][0] = xw[base + o0];
-                        xv[u][1] = xw[base + o1];
-                        pp[u][0] = pv[base + o0];
-                        pp[u][1] = pv[base + o1];
-                        qq[u][0] = Apv[base + o0];
-                        qq[u][1] = Apv[base + o1];
-                    }
+        for (int u = 0; u < kFdLoads; u++) {
+            const int p = p0 + u * xs;
+            if (p < end) {
+                const int o0 = (2 * p) * nx + xc, o1 = o0 + nx;
+                rv[u][0] = rb[o0];
+                rv[u][1] = rb[o1];
+                if (xw) {
+                    xv[u][0] = xw[base + o0];
+                    xv[u][1] = xw[base + o1];
+                    pp[u][0] = pv[base + o0];
+                    pp[u][1] = pv[base + o1];
+                    qq[u][0] = Apv[base + o0];
+                    qq[u][1] = Apv[base + o1];
                 }
             }
+        }
+        if (xw && q0 == P.p0) {  // alpha, while the first loads are on their way
+            if (threadIdx.x < 32) {
+                const float v = cg_alpha(pap, SC, b, kit);
+                if (threadIdx.x == 0) s_a = v;
+            }
+            __syncthreads();
+            a = s_a;
+        }
 #pragma unroll
-            for (int u = 0; u < kFdLoads; u++) {
-                const int p = p0 + u * xs;
-                if (p < P.p1) {
-                    const int o0 = (2 * p) * nx + xc, o1 = o0 + nx;
-                    float r0 = rv[u][0], r1 = rv[u][1];
-                    if (xw) {
-                        xw[base + o0] = xv[u][0] + a * pp[u][0];
-                        xw[base + o1] = xv[u][1] + a * pp[u][1];
-                        r0 -= a * qq[u][0];
-                        r1 -= a * qq[u][1];
-                        rb[o0] = r0;
-                        rb[o1] = r1;
-                        rv[u][0] = r0;
-                        rv[u][1] = r1;
-                    }
-                    R[(p - P.p0) * nx + xc] = make_float2(r0, r1);
+        for (int u = 0; u < kFdLoads; u++) {
+            const int p = p0 + u * xs;
+            if (p < end) {
+                const int o0 = (2 * p) * nx + xc, o1 = o0 + nx;
+                float r0 = rv[u][0], r1 = rv[u][1];
+                if (xw) {
+                    xw[base + o0] = xv[u][0] + a * pp[u][0];
+                    xw[base + o1] = xv[u][1] + a * pp[u][1];
+                    r0 -= a * qq[u][0];
+                    r1 -= a * qq[u][1];
+                    rb[o0] = r0;
+                    rb[o1] = r1;
+                    rv[u][0] = r0;
+                    rv[u][1] = r1;
                 }
+                R[(p - P.p0) * nx + xc] = make_float2(r0, r1);
             }
         }
     }
