@@ -235,6 +235,81 @@ k_mvm_rows(const typename Elem<DT>::T *__restrict__ M, long ldm, const float *__
                 if (b0 + b < nbatch) part[((size_t)ks * nbatch + b0 + b) * nact + r0 + q * kRowThreads] = acc[q][b];
 }
 
+// Products whose split-K grid would leave SMs empty: `wpr` warps of a CTA share
+// one row over all columns, so a few hundred rows fill the chip and the CTA
+// finishes its rows itself (no partial sums in memory, no second launch).  The
+// gradients of NB instances are staged kGvCols columns at a time, with a warp's
+// first loads of M on their way before them.  out[b][row], scale as
+// k_mvm_reduce.  grid: (ceil(nact / (8 / wpr)), ceil(nbatch / NB)).
+// 476 x 2,656 FP32, one instance: 5.0 us, where the split kernel's 30 CTAs took
+// 8.0 and the sum of the splits 1.9 (13.0 -> 8.3 us per call).
+constexpr int kGvWarps = kMvmThreads / 32;
+__host__ __device__ constexpr int gv_cols(int nb) { return nb == 1 ? 4096 : 2048; }
+
+template <int DT, int NB>
+__global__ void __launch_bounds__(kMvmThreads)
+k_mvm_gemv(const typename Elem<DT>::T *__restrict__ M, long ldm, const float *__restrict__ g, long ngrad,
+           const float *__restrict__ scale, float *__restrict__ out, int nact, int nbatch, int wpr) {
+    using E = Elem<DT>;
+    constexpr int V = E::kVec, kCols = gv_cols(NB), kAhead = 4;  // 16-byte loads of a lane in flight
+    __shared__ float4 sg4[NB * kCols / 4];
+    __shared__ float s_sum[kGvWarps][NB];
+    float *sg = reinterpret_cast<float *>(sg4);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, b0 = blockIdx.y * NB;
+    const int row = blockIdx.x * (kGvWarps / wpr) + warp / wpr;
+    const typename E::T *mrow = M + (size_t)min(row, nact - 1) * ldm;
+    const int first = (warp % wpr * 32 + lane) * V, step = wpr * 32 * V;
+    float acc[NB];
+#pragma unroll
+    for (int b = 0; b < NB; b++) acc[b] = 0.f;
+    for (long k0 = 0; k0 < ngrad; k0 += kCols) {
+        const int kn = (int)(ngrad - k0 < kCols ? ngrad - k0 : kCols), kv = (kn + V - 1) / V * V;  // kv <= ldm - k0
+        uint4 raw[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; u++)
+            if (first + u * step < kv) raw[u] = *reinterpret_cast<const uint4 *>(mrow + k0 + first + u * step);
+        for (int i = threadIdx.x; i < NB * kCols; i += kMvmThreads) {
+            const int b = i / kCols, k = i - b * kCols;
+            if (k < kv) sg[i] = b0 + b < nbatch && k < kn ? g[(size_t)(b0 + b) * ngrad + k0 + k] : 0.f;
+        }
+        __syncthreads();
+        for (int c = first; c < kv; c += kAhead * step) {
+#pragma unroll
+            for (int u = 0; u < kAhead; u++) {
+                const int cu = c + u * step;
+                if (cu >= kv) break;
+                float v[V];
+                E::from_raw(raw[u], v);
+                const int next = cu + kAhead * step;
+                if (next < kv) raw[u] = *reinterpret_cast<const uint4 *>(mrow + k0 + next);
+#pragma unroll
+                for (int b = 0; b < NB; b++) {
+#pragma unroll
+                    for (int e = 0; e < V; e += 4) {
+                        const float4 q = sg4[(b * kCols + cu + e) / 4];
+                        acc[b] += v[e] * q.x + v[e + 1] * q.y + v[e + 2] * q.z + v[e + 3] * q.w;
+                    }
+                }
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int b = 0; b < NB; b++) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc[b] += __shfl_xor_sync(0xffffffffu, acc[b], o);
+        if (lane == 0) s_sum[warp][b] = acc[b];
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < kGvWarps / wpr * NB; e += kMvmThreads) {
+        const int r = e / NB, b = e - r * NB, at = blockIdx.x * (kGvWarps / wpr) + r;
+        if (at >= nact || b0 + b >= nbatch) continue;
+        float t = 0.f;
+        for (int q = 0; q < wpr; q++) t += s_sum[r * wpr + q][b];
+        out[(size_t)(b0 + b) * nact + at] = scale ? t * scale[at] : t;
+    }
+}
+
 // out[b][row] = scale[row] * sum_ks part[ks][b][row]
 __global__ void k_mvm_reduce(const float *__restrict__ part, const float *__restrict__ scale,
                              float *__restrict__ out, int nact, int nbatch, int nks) {
@@ -277,6 +352,20 @@ struct Mvm {
         }
         const dim3 grid(NB >= 4 ? (nact + kRowThreads * kRT - 1) / (kRowThreads * kRT) : (nact + kRows - 1) / kRows,
                         nks);
+        // CTAs short of one (register-tiled) or two (streaming) per SM: rows over warps instead
+        if (grid.x * grid.y < (NB >= 4 ? 148u : 2u * 148u)) {
+            constexpr int B = NB >= 4 ? 4 : NB;
+            const int groups = (nbatch + B - 1) / B;
+            int wpr = 1;
+            while (wpr < kGvWarps && (long)nact * wpr * groups < 2L * 148 * kGvWarps &&
+                   2L * wpr * 32 * Elem<DT>::kVec <= ngrad)
+                wpr *= 2;
+            k_mvm_gemv<DT, B><<<dim3((unsigned)((nact * wpr + kGvWarps - 1) / kGvWarps), groups), kMvmThreads, 0, s>>>(
+                reinterpret_cast<const typename Elem<DT>::T *>(m.p), ldm, dg, ngrad,
+                dtype == MB_MVM_FP8 ? scale.p : nullptr, dout, nact, nbatch, wpr);
+            MB_CHECK_LAUNCH();
+            return;
+        }
         const int threads = NB >= 4 ? kRowThreads : kMvmThreads;
         for (int b0 = 0; b0 < nbatch; b0 += NB) {
             kern<<<grid, threads, smem, s>>>(reinterpret_cast<const typename Elem<DT>::T *>(m.p), ldm, dg, ngrad,

@@ -79,3 +79,26 @@ def test_tensor_core_mvm_wide_dynamic_range(dtype):
     for b in range(1, nbatch):
         err = np.linalg.norm(out[b] - want[b]) / np.linalg.norm(want[b])
         assert err < 1e-5, (b, err)
+
+
+@pytest.mark.parametrize("dtype", [0, 1, 2])
+@pytest.mark.parametrize("nact, ngrad, nbatch", [(1, 1, 1), (3, 129, 2), (476, 2656, 1), (300, 4097, 1), (301, 4096, 2),
+                                                 (153, 9001, 1), (2500, 33, 1), (577, 2049, 3)])
+def test_small_mvm_matches_rounded_product(dtype, nact, ngrad, nbatch):
+    """Products too small for the split-K grid (rows shared by warps): one
+    column, one step of staged columns and one past it, several steps, rows that
+    do not fill the last CTA, odd instance strides."""
+    from maos_b200 import native
+    lib = native.load()
+    rng = np.random.default_rng(nact + ngrad)
+    M = rng.standard_normal((nact, ngrad))
+    g = rng.standard_normal((nbatch, ngrad))
+    h = C.c_void_p()
+    native.check(lib.mb_mvm_create(np.asfortranarray(M).ctypes.data_as(C.POINTER(C.c_double)), nact, ngrad, dtype,
+                                   nbatch, C.byref(h)), "mb_mvm_create")
+    out = np.empty((nbatch, nact))
+    native.check(lib.mb_recon_mvm(h, g.ctypes.data_as(C.POINTER(C.c_double)),
+                                  out.ctypes.data_as(C.POINTER(C.c_double))), "mb_recon_mvm")
+    lib.mb_mvm_free(h)
+    want = g.astype(np.float32).astype(np.float64) @ rounded(M, dtype).T
+    assert np.linalg.norm(out - want) / np.linalg.norm(want) < 1e-5
