@@ -31,8 +31,8 @@
 //
 // Every point of every window (the dense kernel for all) was issue-bound at
 // 1,542 us for 8 instances of the 30 m system (6 WFS x 2,820 subapertures, 7
-// layers + 2 DMs); by structure it takes 159 us, and one 8 m LTAO instance 6.8
-// instead of 17 us.
+// layers + 2 DMs); by structure it takes 110 us (159 with the pixel weights
+// formed pixel by pixel), and one 8 m LTAO instance 6.7 instead of 17 us.
 //
 // Stencils are shared by all subapertures with the same amplitude
 // neighbourhood.  The noise is two standard normals per subaperture from a
@@ -165,7 +165,7 @@ __device__ __forceinline__ void geom_store(const GeomWfsT &W, int isa, int iw, i
 struct SepShared {
     int i0[kGeomMaxScr][kSepVec];
     float f0[kGeomMaxScr][kSepVec];
-    float2 w[kGeomMaxScr][kSepVec][kSepPix];  // (average, difference) pixel weights
+    float2 w[kGeomMaxScr][kSepVec][kSepPix + 1];  // (average, difference) pixel weights; odd stride: no conflicts
     float prof[4][kGeomMaxW];
 };
 struct SparseShared {
@@ -174,8 +174,8 @@ struct SparseShared {
 };
 
 // One tile of the separable subapertures (kSepThreads threads).  The pixel
-// weights of an axis are sums of the profile over the window's points,
-// tent-weighted; a subaperture then needs nbu x nbv pixels of each map, split
+// weights of an axis are sums of the profile over the window's points, by a
+// thread per (map, column or row); a subaperture then needs nbu x nbv pixels of each map, split
 // over two threads by rows.  The block's first pixel is subtracted from the
 // others (its share is the stencil's response to a constant, 0 for a gradient)
 // so that the differences, not the OPD itself, meet FP32 rounding.
@@ -188,6 +188,7 @@ __device__ __forceinline__ void sep_tile(const GeomTab &t, const GeomLists &L, S
     const int tt = L.tile[W.tile_off + tile];
     const int c0 = (tt & 0xffff) * kSepTile, r0 = (tt >> 16) * kSepTile;
     for (int e = threadIdx.x; e < 4 * wn; e += kSepThreads) sh.prof[e / wn][e % wn] = L.prof[W.prof_off + e];
+    __syncthreads();
     for (int e = threadIdx.x; e < t.nscr * kSepVec; e += kSepThreads) {
         const int s = e / kSepVec, v = e - s * kSepVec;
         const bool isx = v < kSepTile;
@@ -199,28 +200,37 @@ __device__ __forceinline__ void sep_tile(const GeomTab &t, const GeomLists &L, S
             const double2 w = wind_px[(long)inst * t.natm + s];
             shift = (isx ? w.x : w.y) * (double)isim;
         }
-        geom_base(t.s[s], g0, isx ? c.sx : c.sy, isx ? c.bx : c.by, shift, isx ? t.s[s].nx : t.s[s].ny, sh.i0[s][v],
-                  sh.f0[s][v]);
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < t.nscr * kSepVec * kSepPix; e += kSepThreads) {
-        const int s = e / (kSepVec * kSepPix), v = (e / kSepPix) % kSepVec, b = e % kSepPix;
-        const bool isx = v < kSepTile;
-        const float step = (float)(isx ? t.c[iw][s].sx : t.c[iw][s].sy), f0 = sh.f0[s][v];
-        const int n = isx ? t.s[s].nx : t.s[s].ny, pb = sh.i0[s][v] + b;
-        // points between pixels pb and pb + 1, and pb - 1 and pb, count on the map only
-        const float hi = t.s[s].wrap || (pb >= 0 && pb < n) ? 1.f : 0.f;
-        const float lo = t.s[s].wrap || (pb >= 1 && pb <= n) ? 1.f : 0.f;
+        const int n = isx ? t.s[s].nx : t.s[s].ny;
+        int i0;
+        float f0;
+        geom_base(t.s[s], g0, isx ? c.sx : c.sy, isx ? c.bx : c.by, shift, n, i0, f0);
+        sh.i0[s][v] = i0;
+        sh.f0[s][v] = f0;
+        // walk the window's points: each counts for the pixel before it and the
+        // next (points move less than a pixel), complete once the walk passes it
+        const float step = (float)(isx ? c.sx : c.sy);
         const float *pa = sh.prof[isx ? 2 : 0], *pd = sh.prof[isx ? 1 : 3];
-        float wa = 0.f, wd = 0.f;
-        const float fb = (float)b;
-        for (int c = 0; c < wn; c++) {
-            const float d = fmaf((float)c, step, f0) - fb;  // from the pixel, in pixels
-            const float tent = d >= 0.f ? (d < 1.f ? hi * (1.f - d) : 0.f) : (d > -1.f ? lo * (1.f + d) : 0.f);
-            wa = fmaf(pa[c], tent, wa);
-            wd = fmaf(pd[c], tent, wd);
+        float2 *w = sh.w[s][v];
+        float2 w0 = make_float2(0.f, 0.f), w1 = w0;
+        int k = 0;
+        for (int p = 0; p < wn; p++) {
+            const float u = fmaf((float)p, step, f0), fl = floorf(u);
+            if ((int)fl > k) {
+                w[k++] = w0;
+                w0 = w1;
+                w1 = make_float2(0.f, 0.f);
+            }
+            if (t.s[s].wrap || (i0 + k >= 0 && i0 + k < n)) {  // off the map: no contribution
+                const float a1 = u - fl, a0 = 1.f - a1;
+                w0.x = fmaf(pa[p], a0, w0.x);
+                w0.y = fmaf(pd[p], a0, w0.y);
+                w1.x = fmaf(pa[p], a1, w1.x);
+                w1.y = fmaf(pd[p], a1, w1.y);
+            }
         }
-        sh.w[s][v][b] = make_float2(wa, wd);
+        w[k] = w0;
+        w[k + 1] = w1;
+        for (int q = k + 2; q < kSepPix; q++) w[q] = make_float2(0.f, 0.f);
     }
     __syncthreads();
     const int h = threadIdx.x & 1, sub = threadIdx.x >> 1;
