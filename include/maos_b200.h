@@ -257,10 +257,10 @@ const float *mb_fit_solution(mb_recon *r);
  * a per-member argument table; each member's CG vector updates,
  * preconditioner and fit run between them, members overlapping.  A member's
  * result equals its own mb_recon_step_device's.  Members must share the
- * device and the tomography iteration count; at creation their padded list
- * widths are made equal (exact zeros added; their own graphs are
- * recaptured).  A member stays owned by the caller and must outlive the
- * group; after a member's tables change (updates, autotune) the next step
+ * device and the tomography iteration count (a grouped launch of the layer
+ * kernel holds the members with equal layer rows per thread).  A member stays
+ * owned by the caller and must outlive the group; after a member's tables
+ * change (updates, autotune) the next step
  * recaptures the group's graph.  At most 8 members per grouped launch (more
  * members take more launches). */
 typedef struct mb_group mb_group;
@@ -311,7 +311,7 @@ int mb_recon_serve_step(mb_recon *r, const int *active, const float *grad, float
 /* Autotuner (no counterpart in the reference): times the tomography
  * operator with each admissible row blocking of its pupil-grid kernel (4, 8,
  * 16 pupil rows per CTA, and every even split of the pupil rows into blocks
- * of 1 to 32 rows) and the y-half kernel's CTA size (256, 128 or 64 threads)
+ * of 1 to 32 rows) and the layer kernel's rows per thread (1, 2 or 4)
  * on this batch size, keeps the fastest, then times whole
  * tomography steps with each form of the FDPCG preconditioner
  * (mb_fdpcg_mode; the three-kernel form at each batch shape of
@@ -331,7 +331,8 @@ int mb_autotune(mb_recon *r, int reps, int *rows, float *ms);
  * layers of an instance are split over one thread-block cluster of up to 16
  * CTAs that exchange rows, columns and block members through distributed
  * shared memory, 0 = 2 when that cluster fits on the device, -1 = no change
- * (query).  Results agree to FP32 rounding.  The step graphs are captured
+ * (query).  Without either call: 2 where the cluster fits and all instances'
+ * clusters together have at most 96 CTAs, else 1.  Results agree to FP32 rounding.  The step graphs are captured
  * again.  Returns the form in use (1 or 2) or a negative MB_E* code. */
 int mb_fdpcg_mode(mb_recon *r, int mode);
 
