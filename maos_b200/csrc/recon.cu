@@ -2238,14 +2238,14 @@ void Recon::run_graph(cudaStream_t s) {
 // ---------------------------------------------------------------------------
 // ReconGroup: reconstructors of different geometries (uneven instances)
 // stepped together in one graph.  The tomography operators -- the RHS and
-// every CG iteration's A p (k_pupil_rows: Hx, GP, NEA, GP^T, x half of Hx^T;
-// k_hxt_rows: y half of Hx^T, L2, p.Ap and alpha) -- are one launch for all
+// every CG iteration's A p (k_pupil_rows: Hx, GP, NEA, GP^T; k_hxt_rows:
+// Hx^T, L2 and the p.Ap partials) -- are one launch for all
 // members (GroupTab: per-member arguments and block ranges); each member's
 // own CG vector updates, preconditioner and DM fit run between them on the
 // member's side stream, so those of different members overlap.  Every
 // member's arithmetic is that of its own step, so a member's result is the
-// same in the group as alone.  Members share the CG iteration count; their
-// padded list widths are made equal (the padding adds exact zeros).
+// same in the group as alone.  Members share the CG iteration count; a grouped
+// k_hxt_rows holds the members with equal layer rows per thread.
 // ---------------------------------------------------------------------------
 struct ReconGroup {
     std::vector<Recon *> m;
