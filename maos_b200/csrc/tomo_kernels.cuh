@@ -1791,6 +1791,14 @@ k_fd_data(FdGeomDev G, const int4 *__restrict__ mem, const int2 *__restrict__ bl
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// A barrier in two halves.  A CTA may touch a peer's shared memory only once
+// every CTA of the cluster has started: arriving at kernel entry (nothing is
+// published yet: relaxed) and waiting before the first access hides the wait
+// behind what lies between.
+__device__ __forceinline__ void cluster_arrive_relaxed() {
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
 __device__ __forceinline__ double dsm_peer_f64(const double *local, unsigned rank) {
     unsigned ra;
@@ -2134,10 +2142,11 @@ k_fd_inv(const cplx *__restrict__ H, const float *__restrict__ r, float *__restr
 // CTA owns a range of row pairs and a range of half-spectrum columns of its
 // layer.  Phases, separated by cluster barriers, with the data exchanged
 // through distributed shared memory (ld/st.shared::cluster):
-//   F1  x += a p, r -= a Ap on its row pairs (the CG update, when ab is set),
+//   F1  x += a p, r -= a Ap on its row pairs (the CG update, when xw is set),
 //       row FFTs of r, unpacking into half-spectrum rows stored straight into
 //       the column owners' SC (stores into the receiver's shared memory before
-//       the barrier: no remote load waits on a round trip);
+//       the barrier: no remote load waits on a round trip), once a barrier
+//       entered at the start says that every CTA runs;
 //   F2  column FFTs (SC);
 //   M   its share of the frequency blocks: members gathered from the column
 //       owners' SC, Y = Mbinv X, each stored bin written into its owner's SY;
@@ -2210,6 +2219,7 @@ k_fd_fused(float *__restrict__ r, const __grid_constant__ FdTab ft, const __grid
     pdl_enter();
     // an instance's CTAs are one cluster: all return or none does
     if (inactive(act, blockIdx.y)) return;
+    cluster_arrive_relaxed();  // this CTA has started
     extern __shared__ cplx fsm[];
     __shared__ double sh[32];
     const FdPart P = fu.c[blockIdx.x];
@@ -2282,6 +2292,7 @@ k_fd_fused(float *__restrict__ r, const __grid_constant__ FdTab ft, const __grid
     }
     __syncthreads();
     fft_dir_inplace<true>(L.px, R, S, nx, npr, nx, L.rx, L.nrx, twx, false);
+    cluster_wait();  // B0: every CTA has started, its SC can be stored to
     {  // unpack into half-spectrum rows, each bin stored straight into its
        // column owner's SC (distributed shared memory: stores, no round trip)
         const int hs_ = blockDim.x / h, h0 = threadIdx.x / h, k = threadIdx.x - h0 * h;
