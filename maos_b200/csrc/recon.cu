@@ -1093,9 +1093,8 @@ void Recon::build_fdpcg(const mb_fdpcg_desc *fd) {
     for (int l = 0; l < nps; l++) fdtab.l[l] = fl[l];
     fd_tw.upload(tw);
     MB_REQUIRE(fd_smem <= 200 * 1024, "fdpcg: layer FFT needs %zu bytes of shared memory", fd_smem);
-    MB_CUDA_TRY(cudaFuncSetAttribute(fd_fwd_kern(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fd_smem));
-    for (bool pu : {false, true})
-        MB_CUDA_TRY(cudaFuncSetAttribute(fd_inv_kern(pu), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fd_smem));
+    allow_smem(fd_fwd_kern(), fd_smem);
+    for (bool pu : {false, true}) allow_smem(fd_inv_kern(pu), fd_smem);
     // the CG step's inverse runs as clusters of the group CTAs of an instance when such a cluster fits
     fd_cluster = false;
     if (fdtab.ng <= 16) {
@@ -1232,7 +1231,7 @@ void Recon::build_fdpcg_fused(const std::vector<FdIndex> &idx, const std::vector
             return;
         }
     }
-    MB_CUDA_TRY(cudaFuncSetAttribute(k_fd_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fd_fsmem));
+    allow_smem(k_fd_fused, fd_fsmem);
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = (unsigned)C;

@@ -89,3 +89,44 @@ def test_group_follows_a_member_table_update(group):
     alone = _commands(rs)
     for i in range(len(rs)):
         assert np.array_equal(alone[i], together[i])
+
+
+def test_a_smaller_system_built_later_leaves_the_larger_usable():
+    """The dynamic shared memory a kernel may take belongs to the kernel, which
+    every reconstructor shares.  A 39 m system's layer transforms take nearly
+    twice what a 30 m one's do: built after it, the 30 m one must not take the
+    39 m one's away, in either form of the preconditioner, nor in a group of
+    both."""
+    from conftest import get_fit_assembled, get_system
+    from maos_b200.recon import Reconstructor, ReconGroup
+    rng = np.random.default_rng(21)
+    rs, gs = [], []
+
+    def alone(i, mode):
+        assert rs[i].fdpcg_mode(mode) == mode  # captures the step again
+        rs[i].reset()
+        rs[i].step_device(gs[i].data_ptr())
+        return _commands([rs[i]])[0]
+
+    try:
+        for name in ("elt_39m", "mcao_30m"):
+            s = get_system(name)
+            rs.append(Reconstructor(s, nbatch=1, maxit=3, fit=get_fit_assembled(name)))
+            gs.append(torch.as_tensor(rng.standard_normal((1, s.ngrad)) * 1e-6, dtype=torch.float32, device="cuda"))
+            if len(rs) == 1:
+                before = {mode: alone(0, mode) for mode in (1, 2)}
+        for mode in (1, 2):
+            want = [alone(i, mode) for i in range(2)]
+            assert np.array_equal(want[0], before[mode])
+            G = ReconGroup(rs)
+            try:
+                for R in rs:
+                    R.reset()
+                G.step_device([g.data_ptr() for g in gs])
+                for a, b in zip(_commands(rs), want):
+                    assert np.array_equal(a, b)
+            finally:
+                G.close()
+    finally:
+        for R in rs:
+            R.close()
