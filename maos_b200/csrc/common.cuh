@@ -52,6 +52,8 @@ struct InvalidArg {
         }                                                                                  \
     } while (0)
 
+constexpr int kSms = 148;  // streaming multiprocessors of a B200
+
 // Owning device buffer.
 template <typename T>
 struct DevBuf {

@@ -6,11 +6,14 @@
 // FP32, BF16, or FP8-E4M3 with one FP32 scale per row; accumulation is FP32.
 // A BF16 or FP8 matrix installed for batches of 4 or more is stored instead
 // in the tensor-core tile order of mvm_tc.cuh and multiplied there.
-// The kernel is split-K: CTA (rt, ks) multiplies a tile of kRows rows by a
-// kK-column slab, with that slab of every instance's gradients staged in
-// shared memory, and writes per-split partial sums; a second kernel adds the
-// splits in fixed order and applies the row scale (deterministic, no atomics).
-// Each warp streams rows with 16-byte vector loads, so M is read exactly once.
+// The rows are multiplied by one of two forms (gemv_pays chooses):
+//   split-K: CTA (rt, ks) multiplies a tile of rows by a kK-column slab, with
+//   that slab of up to kMaxBatch instances' gradients staged in shared memory,
+//   and writes per-split partial sums; a second kernel adds the splits in fixed
+//   order and applies the row scale (deterministic, no atomics).  Rows are
+//   streamed with 16-byte vector loads; M is read once per 16 instances.
+//   k_mvm_gemv: warps share a row over all columns, one launch; M is read once
+//   per 4 instances.
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
 #include <cuda_runtime.h>
@@ -235,12 +238,15 @@ k_mvm_rows(const typename Elem<DT>::T *__restrict__ M, long ldm, const float *__
                 if (b0 + b < nbatch) part[((size_t)ks * nbatch + b0 + b) * nact + r0 + q * kRowThreads] = acc[q][b];
 }
 
-// Products whose split-K grid would leave SMs empty: `wpr` warps of a CTA share
-// one row over all columns, so a few hundred rows fill the chip and the CTA
-// finishes its rows itself (no partial sums in memory, no second launch).  The
-// gradients of NB instances are staged kGvCols columns at a time, with a warp's
-// first loads of M on their way before them.  out[b][row], scale as
-// k_mvm_reduce.  grid: (ceil(nact / (8 / wpr)), ceil(nbatch / NB)).
+// Small products: `wpr` warps of a CTA share one row over all columns, so a few
+// hundred rows fill the chip and the CTA finishes its rows itself (no partial
+// sums in memory, no second launch).  The gradients of NB instances are staged
+// gv_cols columns at a time, with a warp's first loads of M on their way before
+// them; each stage is a serial step of the CTA, which bounds how many columns
+// pay (gemv_pays).  out[b][row], scale as k_mvm_reduce.  Relative error against
+// 64 bits, mean of 24 products: 476 x 2,656 FP32 9.9e-8 (split-K 1.06e-7), 8
+// instances 9.5e-8 (7.4e-7).
+// grid: (ceil(nact / (8 / wpr)), ceil(nbatch / NB)).
 // 476 x 2,656 FP32, one instance: 5.0 us, where the split kernel's 30 CTAs took
 // 8.0 and the sum of the splits 1.9 (13.0 -> 8.3 us per call).
 constexpr int kGvWarps = kMvmThreads / 32;
@@ -310,6 +316,54 @@ k_mvm_gemv(const typename Elem<DT>::T *__restrict__ M, long ldm, const float *__
     }
 }
 
+// Warps per row of k_mvm_gemv for `groups` groups of instances: until two CTAs
+// per SM have rows, or a lane has fewer than two loads.
+template <int DT>
+static int gemv_warps(int nact, long ngrad, int groups) {
+    int wpr = 1;
+    while (wpr < kGvWarps && (long)nact * wpr * groups < 2L * kSms * kGvWarps &&
+           2L * wpr * 32 * Elem<DT>::kVec <= ngrad)
+        wpr *= 2;
+    return wpr;
+}
+
+// Whether k_mvm_gemv<DT, min(NB, 4)> is the faster form for this product, from
+// 586 shapes of 100 to 9,900 rows and 200 to 36,000 columns timed in both forms
+// (the form chosen is nowhere more than 5% slower than the other).
+// One or two instances: the split form's two launches take 10-16 us whatever
+// the shape; the other one about 4 us per stage of columns and 0.6 us per 10^6
+// elements of M.  476 x 2,656 FP32: 6.3 against 12.4 us; 476 x 30,000: 34
+// against 14; 8,000 x 2,000: 14.5 against 14.5.
+// More: k_mvm_rows takes about the same time for every pass of NB instances,
+// as few CTAs walk kK columns each; k_mvm_gemv takes a fixed time per stage and
+// wave of its CTAs, less where warps share rows.  FP32, 8 instances: 476 x
+// 2,656 16 against 196 us, 5,000 x 8,000 238 against 296, 8,000 x 8,000 329
+// against 284; 64 instances: 8,000 x 16,250 4,832 against 1,375.
+template <int DT, int NB>
+static bool gemv_pays(int nact, long ngrad, int nbatch) {
+    constexpr int B = NB >= 4 ? 4 : NB;
+    const long groups = (nbatch + B - 1) / B, stages = (ngrad + gv_cols(B) - 1) / gv_cols(B);
+    if (groups > 65535) return false;  // grid.y
+    if constexpr (NB < 4) {
+        constexpr double kLaunches = DT == MB_MVM_F32 ? 3.3 : DT == MB_MVM_BF16 ? 2.65 : 2.15;  // worth of two, in stages
+        return (double)stages + 0.15e-6 * (double)nact * (double)ngrad <= kLaunches;
+    } else {
+        static const int resident = [] {  // CTAs on the device at once
+            int n = 0;
+            MB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_mvm_gemv<DT, B>, kMvmThreads, 0));
+            return std::max(1, n) * kSms;
+        }();
+        const int wpr = gemv_warps<DT>(nact, ngrad, (int)groups);
+        // a group with one or two of its four instances takes half as long
+        const double ctas = (double)(((long)nact * wpr + kGvWarps - 1) / kGvWarps) * ((nbatch + 1) / 2) / 2;
+        const double step = DT == MB_MVM_F32 ? 6 + 14.0 / wpr : DT == MB_MVM_BF16 ? 5.5 + 7.5 / wpr : 5.5 + 12.0 / wpr;
+        const double pass = DT == MB_MVM_F32    ? (NB == 4 ? 400 : NB == 8 ? 300 : 345)
+                            : DT == MB_MVM_BF16 ? (nact <= 256 ? 90 : 140)
+                                                : 77;
+        return (double)stages * std::ceil(ctas / resident) * step <= ((nbatch + NB - 1) / NB) * pass;  // us
+    }
+}
+
 // out[b][row] = scale[row] * sum_ks part[ks][b][row]
 __global__ void k_mvm_reduce(const float *__restrict__ part, const float *__restrict__ scale,
                              float *__restrict__ out, int nact, int nbatch, int nks) {
@@ -352,15 +406,10 @@ struct Mvm {
         }
         const dim3 grid(NB >= 4 ? (nact + kRowThreads * kRT - 1) / (kRowThreads * kRT) : (nact + kRows - 1) / kRows,
                         nks);
-        // CTAs short of one (register-tiled) or two (streaming) per SM: rows over warps instead
-        if (grid.x * grid.y < (NB >= 4 ? 148u : 2u * 148u)) {
+        if (gemv_pays<DT, NB>(nact, ngrad, nbatch)) {
             constexpr int B = NB >= 4 ? 4 : NB;
-            const int groups = (nbatch + B - 1) / B;
-            int wpr = 1;
-            while (wpr < kGvWarps && (long)nact * wpr * groups < 2L * 148 * kGvWarps &&
-                   2L * wpr * 32 * Elem<DT>::kVec <= ngrad)
-                wpr *= 2;
-            k_mvm_gemv<DT, B><<<dim3((unsigned)((nact * wpr + kGvWarps - 1) / kGvWarps), groups), kMvmThreads, 0, s>>>(
+            const int groups = (nbatch + B - 1) / B, wpr = gemv_warps<DT>(nact, ngrad, groups);
+            k_mvm_gemv<DT, B><<<dim3((unsigned)(((long)nact * wpr + kGvWarps - 1) / kGvWarps), groups), kMvmThreads, 0, s>>>(
                 reinterpret_cast<const typename Elem<DT>::T *>(m.p), ldm, dg, ngrad,
                 dtype == MB_MVM_FP8 ? scale.p : nullptr, dout, nact, nbatch, wpr);
             MB_CHECK_LAUNCH();
