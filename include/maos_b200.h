@@ -257,11 +257,9 @@ const float *mb_fit_solution(mb_recon *r);
  * a per-member argument table; each member's CG vector updates,
  * preconditioner and fit run between them, members overlapping.  A member's
  * result equals its own mb_recon_step_device's.  Members must share the
- * device and the tomography iteration count (a grouped launch of the layer
- * kernel holds the members with equal layer rows per thread).  A member stays
- * owned by the caller and must outlive the group; after a member's tables
- * change (updates, autotune) the next step
- * recaptures the group's graph.  At most 8 members per grouped launch (more
+ * device and the tomography iteration count.  A member stays owned by the
+ * caller and must outlive the group; after a member's tables change (updates,
+ * autotune) the next step recaptures the group's graph.  At most 8 members per grouped launch (more
  * members take more launches). */
 typedef struct mb_group mb_group;
 int mb_group_create(mb_recon *const *members, int n, mb_group **out);

@@ -566,10 +566,6 @@ static PupilGroupKern pupil_group_kern(bool from_x, bool p2) {
 // and of k_hxt_rows, by the layer rows per thread
 using HxtKern = void (*)(HxtArgs);
 static HxtKern hxt_kern(int rt) { return rt == 4 ? k_hxt_rows<4> : rt == 2 ? k_hxt_rows<2> : k_hxt_rows<1>; }
-using HxtGroupKern = void (*)(GroupTab<HxtArgs>);
-static HxtGroupKern hxt_group_kern(int rt) {
-    return rt == 4 ? k_hxt_rows_group<4> : rt == 2 ? k_hxt_rows_group<2> : k_hxt_rows_group<1>;
-}
 // Allow `smem` bytes of dynamic shared memory; the largest any caller asked
 // for stays allowed (kernels are shared by all reconstructors).
 template <class K>
@@ -714,7 +710,7 @@ void Recon::pupil_rows(bool from_x, const float *xin, cudaStream_t s) {
 HxtArgs Recon::hxt_args(const float *xin, float *out, double *dot_part, int do_l2) const {
     return HxtArgs{obuf.p, xin,    out, dot_part, HxtIndex{hxt_x0.p, hxt_xw.p, hxt_y0.p, hxt_yw.p},
                    hxttab, laytab, nps, nwfs,     orows,
-                   ostride, nxtot, do_l2, act()};
+                   ostride, nxtot, do_l2, hrows,    act()};
 }
 
 void Recon::hxt_rows(const float *xin, float *out, double *dot_part, int do_l2, cudaStream_t s) {
@@ -2243,8 +2239,7 @@ void Recon::run_graph(cudaStream_t s) {
 // own CG vector updates, preconditioner and DM fit run between them on the
 // member's side stream, so those of different members overlap.  Every
 // member's arithmetic is that of its own step, so a member's result is the
-// same in the group as alone.  Members share the CG iteration count; a grouped
-// k_hxt_rows holds the members with equal layer rows per thread.
+// same in the group as alone.  Members share the CG iteration count.
 // ---------------------------------------------------------------------------
 struct ReconGroup {
     std::vector<Recon *> m;
@@ -2320,23 +2315,18 @@ struct ReconGroup {
     }
     void hxt_rows(const std::vector<int> &who, const std::vector<const float *> &xin, const std::vector<float *> &out,
                   const std::vector<double *> &dot, int do_l2, cudaStream_t s) {
-        for (int rt : {1, 2, 4}) {
-            std::vector<int> b;
-            for (int i : who)
-                if (m[i]->hrows == rt) b.push_back(i);
-            for (size_t c0 = 0; c0 < b.size(); c0 += kMaxGroup) {
-                GroupTab<HxtArgs> g{};
-                g.n = (int)std::min(b.size() - c0, (size_t)kMaxGroup);
-                g.start[0] = 0;
-                for (int e = 0; e < g.n; e++) {
-                    const int i = b[c0 + e];
-                    const Recon &R = *m[i];
-                    g.a[e] = R.hxt_args(xin[i], out[i], dot[i], do_l2);
-                    g.grid[e] = make_uint3((unsigned)R.nblk_hxt, (unsigned)R.nb, 1u);
-                    g.start[e + 1] = g.start[e] + g.grid[e].x * g.grid[e].y;
-                }
-                launch(hxt_group_kern(rt), dim3(g.start[g.n]), dim3(kHxtThreads), 0, s, g);
+        for (size_t c0 = 0; c0 < who.size(); c0 += kMaxGroup) {
+            GroupTab<HxtArgs> g{};
+            g.n = (int)std::min(who.size() - c0, (size_t)kMaxGroup);
+            g.start[0] = 0;
+            for (int e = 0; e < g.n; e++) {
+                const int i = who[c0 + e];
+                const Recon &R = *m[i];
+                g.a[e] = R.hxt_args(xin[i], out[i], dot[i], do_l2);
+                g.grid[e] = make_uint3((unsigned)R.nblk_hxt, (unsigned)R.nb, 1u);
+                g.start[e + 1] = g.start[e] + g.grid[e].x * g.grid[e].y;
             }
+            launch(k_hxt_rows_group, dim3(g.start[g.n]), dim3(kHxtThreads), 0, s, g);
         }
     }
     // A p for every member (TomoL): grouped where the tip/tilt split allows

@@ -706,7 +706,7 @@ struct HxtArgs {
     LayerTab lt;
     int nps, nwfs, orows, ostride;  // rows of a WFS's plane of o, and their stride
     long nxtot;
-    int do_l2;
+    int do_l2, rt;  // rt: the layer rows per thread the tables were built for
     const int *act;
 };
 
@@ -864,11 +864,15 @@ template <int RT>
 __global__ void __launch_bounds__(kHxtThreads) k_hxt_rows(const __grid_constant__ HxtArgs a) {
     hxt_rows_body<RT>(blockIdx, gridDim.x, a);
 }
-template <int RT>
+// The members' rows per thread may differ (a CTA serves one member).
 __global__ void __launch_bounds__(kHxtThreads) k_hxt_rows_group(const __grid_constant__ GroupTab<HxtArgs> g) {
     uint3 bid;
     const int e = group_entry(g, bid);
-    hxt_rows_body<RT>(bid, g.grid[e].x, g.a[e]);
+    switch (g.a[e].rt) {
+        case 1: hxt_rows_body<1>(bid, g.grid[e].x, g.a[e]); break;
+        case 2: hxt_rows_body<2>(bid, g.grid[e].x, g.a[e]); break;
+        default: hxt_rows_body<4>(bid, g.grid[e].x, g.a[e]); break;
+    }
 }
 
 // ---------------------------------------------------------------------------

@@ -91,6 +91,44 @@ def test_group_follows_a_member_table_update(group):
         assert np.array_equal(alone[i], together[i])
 
 
+def test_one_launch_per_operator_whatever_the_rows_per_thread():
+    """Members whose layer kernels keep 1 (2 instances of the 8 m system), 2 and
+    4 layer rows per thread (6 and 23 of the 30 m one) share one launch of it:
+    bit for bit the members' own results, and for every application of an
+    operator (the right-hand side, A x, A p of each iteration) one launch of
+    each kernel instead of one per member."""
+    from conftest import get_fit_assembled, get_system
+    from maos_b200.recon import Reconstructor, ReconGroup
+    rng = np.random.default_rng(22)
+    iters, members = 3, (("scao_8m", 2), ("mcao_30m", 6), ("mcao_30m", 23))
+    rs, gs, pos = [], [], set()
+    try:
+        for name, nb in members:
+            s = get_system(name)
+            pos.add(round(s.wfs[0].dsa / s.pmap.dx))
+            rs.append(Reconstructor(s, nbatch=nb, maxit=iters, fit=get_fit_assembled(name)))
+            gs.append(torch.as_tensor(rng.standard_normal((nb, s.ngrad)) * 1e-6, dtype=torch.float32, device="cuda"))
+        lib = rs[0].lib
+        lib.mb_kernel_launches(1)
+        for R, g in zip(rs, gs):
+            R.step_device(g.data_ptr())
+        n_alone, want = lib.mb_kernel_launches(1), _commands(rs)
+        G = ReconGroup(rs)
+        try:
+            for R in rs:
+                R.reset()
+            G.step_device([g.data_ptr() for g in gs])
+            for a, b in zip(_commands(rs), want):
+                assert np.array_equal(a, b)
+            saved = (len(rs) - len(pos)) + (len(rs) - 1)  # k_pupil_rows: a launch per subaperture/pupil ratio
+            assert G.graph_kernels == n_alone - (iters + 2) * saved
+        finally:
+            G.close()
+    finally:
+        for R in rs:
+            R.close()
+
+
 def test_a_smaller_system_built_later_leaves_the_larger_usable():
     """The dynamic shared memory a kernel may take belongs to the kernel, which
     every reconstructor shares.  A 39 m system's layer transforms take nearly
