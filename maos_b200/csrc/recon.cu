@@ -1072,6 +1072,7 @@ void Recon::build_fdpcg(const mb_fdpcg_desc *fd) {
         for (int g = 0; g < fdtab.ng; g++) {
             const FdLayer &F = fl[fdtab.g[g].l[0]];
             const int n = fdtab.g[g].n;
+            if (n == 1) fdtab.g[g].inv_np2 = 0;  // every row pair is the layer's (the reciprocal is exact to 256 pairs)
             fd_bufn = std::max(fd_bufn, n * std::max(F.ny / 2 * F.nx, F.ny * (F.nx / 2 + 1)));
             if (F.px >= 0) fd_bufn = std::max(fd_bufn, fft2_scratch(F.px, true, n * F.ny / 2));
             if (F.py >= 0) fd_bufn = std::max(fd_bufn, fft2_scratch(F.py, false, n * (F.nx / 2 + 1)));

@@ -1107,7 +1107,7 @@ struct FdLayer {
 // Layers of one size whose transforms a CTA does together.
 struct FdGroup {
     int n;
-    int inv_np2;  // ceil(2^16 / row pairs of a layer): p / np2 = p * inv_np2 >> 16 for the group's row pairs
+    int inv_np2;  // ceil(2^16 / row pairs of a layer): p / np2 = p * inv_np2 >> 16 for the group's row pairs (one layer: 0)
     signed char l[kMaxLayers];
 };
 struct FdTab {  // per layer and group, by value (kernel parameter space)

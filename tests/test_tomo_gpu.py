@@ -246,6 +246,44 @@ def test_fdpcg_batch_shape_keeps_results():
         R.close()
 
 
+def test_layer_transforms_of_a_tall_layer_beside_grouped_ones():
+    """Once an instance's layers outnumber the SMs, equal layers share a CTA of
+    the transforms, which then tells a row pair's layer by a multiplication; a
+    layer of its own must not (its 480 row pairs are past where that is exact).
+    Blocks of one frequency with M = 1 make the preconditioner the identity,
+    whatever the layers' shapes, and the solve the unpreconditioned one."""
+    import dataclasses
+
+    from conftest import get_system
+    from maos_b200.fdpcg_setup import FdpcgTables
+    from maos_b200.geometry import Grid
+    from maos_b200.recon import Reconstructor
+    s = get_system("ltao_8m")
+    dx = s.pmap.dx
+    xmaps = [Grid(nx, ny, dx, dx, -nx / 2 * dx, -ny / 2 * dx, ht)
+             for nx, ny, ht in ((16, 16, 0.0), (16, 960, 1000.0), (16, 16, 2000.0))]
+    n = sum(g.n for g in xmaps)
+    eye = FdpcgTables(bs=1, nb=n, adimx=n, adimy=1, scale=1, perm=np.arange(n), Mbinv=np.ones((n, 1, 1), complex),
+                      nxtot=n)
+    nb = 50  # 150 (layer, instance) planes
+    rng = np.random.default_rng(31)
+    x = rng.standard_normal((nb, n)) * 1e-7
+    g = rng.standard_normal((nb, s.ngrad)) * 1e-6
+    got = []
+    for precond in (1, 0):
+        t = dataclasses.replace(s, xmaps=xmaps, l2c=np.full(3, s.l2c[0]), fdpcg=eye,
+                                cfg=dataclasses.replace(s.cfg, tomo_precond=precond))
+        R = Reconstructor(t, nbatch=nb, maxit=3)
+        try:
+            if precond:
+                R.fdpcg_mode(1)
+                assert rel(R.apply_fdpcg(x), x) < OP_TOL
+            got.append(R.tomo(g)[0])
+        finally:
+            R.close()
+    assert rel(got[0], got[1]) < SOLVE_TOL
+
+
 def test_fused_preconditioner_matches_the_oracle(setup):
     """The fused FDPCG step (mb_fdpcg_mode 2: one cluster kernel per CG step,
     the layers split over its CTAs) solves to the oracle's tolerance, agrees
