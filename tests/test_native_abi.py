@@ -68,3 +68,10 @@ def test_mvm_rejects_bad_arguments(lib):
                                   ctypes.POINTER(ctypes.c_void_p)]
     assert lib.mb_mvm_create(M.ctypes.data_as(P), 2, 2, 7, 1, ctypes.byref(h)) == -1
     assert lib.mb_mvm_create(None, 2, 2, 0, 1, ctypes.byref(h)) == -1
+
+
+def test_a_change_of_any_source_rebuilds_the_library():
+    from maos_b200 import build
+    csrc = os.path.join(build.HERE, "csrc")
+    listed = {os.path.normpath(f) for f in build.SOURCES + build.HEADERS}
+    assert {os.path.join("csrc", f) for f in os.listdir(csrc) if f.endswith((".cu", ".cuh"))} <= listed
