@@ -216,6 +216,11 @@ def run_reference(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
         return 0
+    from oracle import refbridge
+    if not os.path.exists(refbridge.LIB):
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's CPU library is not built: "
+                          "its sources (MAOS_REF, make -C oracle/ref) are not on this machine"}), flush=True)
+        return 0
     from maos_b200 import config, fit_assemble, geometry, turbulence
     sysm = geometry.build_tomo(config.PRESETS[WORKLOAD]())
     fit = fit_assemble.build_fit_assembled(sysm)
