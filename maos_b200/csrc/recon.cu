@@ -496,11 +496,11 @@ void Recon::build_blocking() {
     for (int l = 0; l < nps; l++)
         for (int rt : {1, 2, 4}) orows = std::max(orows, hxt_window(l, rt));
     // pupil rows per CTA: as many row blocks per WFS as one wave of 4 CTAs on
-    // each of 148 SMs holds, at least 3 and with at least 4 rows per block;
+    // each SM holds, at least 3 and with at least 4 rows per block;
     // Recon::autotune replaces the guess by measurement.  Fewer rows where
     // the block's tables would not fit.
     const long nmax = (nyp + 3) / 4;
-    const long tiles = std::max(3L, std::min(nmax, (long)(4 * 148) / std::max(1L, (long)nwfs * nb)));
+    const long tiles = std::max(3L, std::min(nmax, (long)(4 * kSms) / std::max(1L, (long)nwfs * nb)));
     int rows = (int)((nyp + tiles - 1) / tiles);
     while (rows > 1 && pupil_smem_of(rows) > kMaxRowSmem) rows = (rows + 1) / 2;
     if (const char *e = std::getenv("MAOS_B200_PUPIL_ROWS")) {  // tuning override
@@ -515,7 +515,7 @@ void Recon::build_blocking() {
         for (int l = 0; l < nps; l++) n += (long)((lay_h[l].ny + rt - 1) / rt) * lay_h[l].nx;
         return n * nb;
     };
-    set_hxt_rows(threads(4) >= 148L * 8 * kHxtThreads ? 4 : threads(2) >= 148L * 4 * kHxtThreads ? 2 : 1);
+    set_hxt_rows(threads(4) >= 8L * kSms * kHxtThreads ? 4 : threads(2) >= 4L * kSms * kHxtThreads ? 2 : 1);
 }
 
 // The layer rows that each block of `rows` pupil rows (with its halo)
@@ -1020,7 +1020,7 @@ void Recon::build_fdpcg(const mb_fdpcg_desc *fd) {
         return n == 1;
     };
     fd_bufn = 0;
-    int twn = 0;  // twiddle entries a layer CTA stages (nx + ny)
+    int twn = 0;  // twiddle entries a CTA stages (nx + ny)
     for (int l = 0; l < nps; l++) {
         FdLayer &F = fl[l];
         F.nx = lay_h[l].nx;
@@ -1083,7 +1083,7 @@ void Recon::build_fdpcg(const mb_fdpcg_desc *fd) {
     for (const FdLayer &F : fl) most = std::max(most, (long)F.nx * F.ny);
     constexpr size_t kSmSmem = 227 * 1024, kPerCta = 1024;
     const size_t alone = buffers(0);
-    fd_smem = (long)nb * nps > 148 ? buffers(most) : alone;
+    fd_smem = (long)nb * nps > kSms ? buffers(most) : alone;
     if (fd_smem > 200 * 1024 || kSmSmem / (fd_smem + kPerCta) < std::min<size_t>(2, kSmSmem / (alone + kPerCta)))
         fd_smem = buffers(0);
     fd_lay.upload(fl);
@@ -1115,6 +1115,8 @@ void Recon::build_fdpcg(const mb_fdpcg_desc *fd) {
     }
     build_fdpcg_fused(idx, hoff);
 }
+
+constexpr int kFusedCtas = 96;  // most CTAs of all instances' clusters for which the fused form is the default
 
 // Split each layer over K_l CTAs of an instance's cluster (K_l proportional
 // to its size, at most 16 CTAs in all), the CTAs' row-pair, column and block
@@ -1248,11 +1250,11 @@ void Recon::build_fdpcg_fused(const std::vector<FdIndex> &idx, const std::vector
     fused_tab = T;
     fd_fused_ok = true;
     // the fused form while every instance's cluster runs at once beside the
-    // others: 6 instances of the 30 m system 314 against 364 us per step of 4
+    // others (one CTA per SM, clusters within a GPC: not all 148): 6 instances of the 30 m system 314 against 364 us per step of 4
     // iterations, 8 (two rounds of clusters) 373 against 379; 5 of the 39 m one
     // 569 against 636, 8 731 against 706.  mb_autotune and mb_fdpcg_mode choose
     // otherwise.
-    if (nb * fused_tab.C <= 96) fd_mode = 2;
+    if (nb * fused_tab.C <= kFusedCtas) fd_mode = 2;
 }
 
 // The data term's geometry on the device: per block its base pupil
@@ -1522,7 +1524,7 @@ bool Recon::op_fdpcg(float *rin, float *zout, double *rzp, cudaStream_t s, int k
            pupd, Apupd, PapParts{pap_part.p, nblk_hxt}, scal(), k, act());
     fd_mul(s);
     CgScal S = in_cg ? scal() : CgScal{};
-    if (in_cg && pnext && fd_cluster) {  // the p update inside, clusters of the layer CTAs
+    if (in_cg && pnext && fd_cluster) {  // the p update inside, clusters of an instance's group CTAs
         launch_cluster(fd_inv_kern(true), dim3(fdtab.ng, nb), dim3(kFftThreads), fd_smem, s, fdtab.ng, spec2.p, rin, zout,
                        rzp, fdtab, fd_tw.p, nxtot, fd_bufn, S, k, init, act(), pnext);
         return true;

@@ -285,8 +285,9 @@ __global__ void k_gp(const float *__restrict__ opd, const float *__restrict__ gi
 
 // The p.Ap partials that the operator left, n per instance.  Whoever updates
 // x and r forms alpha from them: the producers need no fence, counter and last
-// block, whose three round trips came after everything else (k_hxt_rows, one 8
-// m LTAO instance 7.2 -> 5.3 us; k_spmv_lr, 32 30 m instances 32 -> 22 us).
+// block, whose three round trips come after everything else (with them and
+// without: k_hxt_rows, one 8 m LTAO instance 7.2 and 5.3 us; k_spmv_lr, 32 30 m
+// instances 32 and 22 us).
 struct PapParts {
     const double *part;  // [b][n]
     int n;
@@ -864,7 +865,9 @@ template <int RT>
 __global__ void __launch_bounds__(kHxtThreads) k_hxt_rows(const __grid_constant__ HxtArgs a) {
     hxt_rows_body<RT>(blockIdx, gridDim.x, a);
 }
-// The members' rows per thread may differ (a CTA serves one member).
+// The members' rows per thread may differ (a CTA serves one member): a launch
+// for each number of rows took the served mix (26 + 26 8 m, 12 30 m instances)
+// 2,823 us per step, one launch takes 2,655.
 __global__ void __launch_bounds__(kHxtThreads) k_hxt_rows_group(const __grid_constant__ GroupTab<HxtArgs> g) {
     uint3 bid;
     const int e = group_entry(g, bid);

@@ -9,7 +9,7 @@ Builds the system, sets up a reconstructor with the DM fit for `batch`
 instances and runs `steps` graph steps on random gradients; prints "ok".
 Under ncu, each step's kernels appear in order: k_gp, k_pupil_rows (right-hand
 side), k_hxt_rows, then per FDPCG iteration k_pupil_rows, k_hxt_rows,
-k_fd_fwd, k_fd_mul, k_fd_inv, k_cg_update_p, then the fit.
+k_fd_fwd, k_fd_mul, k_fd_inv (with the p update), then the fit.
 
 With --wfs, the system's geometric WFS (every WFS, its atmosphere and DMs,
 noise on) runs `steps` times for `batch` instances instead (k_wfs_geom).
@@ -21,7 +21,7 @@ times are printed.
 
 With --mvm, a random control matrix of the system's shape (nact x ngrad) is
 installed in that storage type and `steps` batched MVMs are applied instead
-(k_gsplit, k_mvm_tc, k_mvm_reduce for BF16/FP8 at 4 or more instances).
+(k_gsplit or k_gsplit8 and k_mvm_tc for BF16/FP8 at 4 or more instances).
 """
 from __future__ import annotations
 

@@ -2,8 +2,8 @@
 
 Each row crosses a line of the dispatch: vectors interleaved by 1, 2, 4 or 8
 instances with a partial last group (3, 5, 9), the V'p product with 4 x 4 sums
-per thread (64 and more), one to four layer rows per thread of the y half of
-Hx^T, the preconditioner in one cluster kernel (up to 6 instances of the 30 m
+per thread (64 and more), one to four layer rows per thread of the kernel
+that applies Hx^T, the preconditioner in one cluster kernel (up to 6 instances of the 30 m
 system), in three kernels, and with several layers per CTA (25 instances: 150
 (layer, instance) planes for 148 SMs); the cluster kernel for the vector part of
 an unpreconditioned iteration with 4 elements per thread (8 m, the fits) and 8

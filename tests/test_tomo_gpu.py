@@ -199,9 +199,9 @@ def test_integrated_tip_tilt_split0(name):
 
 def test_autotune_keeps_results():
     """The autotuner changes blockings and launch shapes only: the pupil-row
-    blocking changes no bit; the y-half CTA size changes the order of the
-    FP64 p.Ap partial sums and the preconditioner's form changes FP32
-    rounding, so the solution agrees to FP32 rounding."""
+    blocking changes no bit; the layer kernel's rows per thread change the
+    order of the FP64 p.Ap partial sums and the preconditioner's form changes
+    FP32 rounding, so the solution agrees to FP32 rounding."""
     from conftest import get_system
     from maos_b200.recon import Reconstructor
     s = get_system("mcao_30m")
