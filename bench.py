@@ -322,7 +322,7 @@ def wfs_rates(sysm, fit, batch: int, stream, cpu: bool = True):
     nmap = len(sysm.cfg.atm_ht) + len(fit.dms)
     res = {"instances": batch, "ms": ms, "steps_per_s": batch * 1000.0 / ms, "kernel": "k_wfs_geom",
            "wfs": geom.nwfs, "subapertures": int(sum(len(p.ix0) for p in P)), "points_per_subaperture_side": P[0].nxsa,
-           "maps": nmap, "interpolations_per_s": pts * nmap * batch / (ms / 1000.0),
+           "maps": nmap, "window_points_times_maps_per_s": pts * nmap * batch / (ms / 1000.0),
            "data": "seeded von Karman layers (4 seeds over the instances), random DM commands, noise on"}
     W.close()
     if cpu:
