@@ -134,8 +134,10 @@ struct Recon {
 
     // tables
     RayTables hx;
-    // k_pupil_rows: pupil rows per CTA, CTAs per WFS, the layer rows each touches
+    // k_pupil_rows: pupil rows per CTA, CTAs per WFS, the layer rows each touches;
+    // whether it also forms the LHS's Hx and gradients (op_lhs)
     int prows = 0, ptiles = 0, pvrows = 0;
+    bool lhs_fused = false;
     size_t pupil_smem = 0;
     DevBuf<int2> vrow;
     // k_hxt_rows: layer rows per thread, CTAs per instance, the transposed lists as windows
@@ -294,10 +296,11 @@ struct Recon {
     void set_hxt_rows(int rows);
     void rebuild_fdpcg_device();
     int autotune(int reps, float *ms_out);
-    void pupil_rows(bool from_x, const float *xin, cudaStream_t s);
+    void pupil_rows(bool from_x, const float *xin, cudaStream_t s, bool tt = true);
+    void lhs_pupil(const float *xin, cudaStream_t s);
     void hxt_rows(const float *xin, float *out, double *dot_part, int do_l2, cudaStream_t s);
     // the arguments of those launches (also gathered by a ReconGroup)
-    PupilArgs pupil_args(bool from_x, const float *xin, int w0) const;
+    PupilArgs pupil_args(bool from_x, const float *xin, int w0, bool tt = true) const;
     HxtArgs hxt_args(const float *xin, float *out, double *dot_part, int do_l2) const;
     void build_wfs_tables(const mb_recon_desc *d);
     void build_fdpcg(const mb_fdpcg_desc *fd);
@@ -498,7 +501,10 @@ void Recon::build_blocking() {
     // pupil rows per CTA: as many row blocks per WFS as one wave of 4 CTAs on
     // each SM holds, at least 3 and with at least 4 rows per block;
     // Recon::autotune replaces the guess by measurement.  Fewer rows where
-    // the block's tables would not fit.
+    // the block's tables would not fit; where not even one row's do (many layers
+    // much finer than the pupil), Hx and the gradients go through memory.
+    lhs_fused = split != 0;
+    if (lhs_fused && pupil_smem_of(1) > kMaxRowSmem) lhs_fused = false;
     const long nmax = (nyp + 3) / 4;
     const long tiles = std::max(3L, std::min(nmax, (long)(4 * kSms) / std::max(1L, (long)nwfs * nb)));
     int rows = (int)((nyp + tiles - 1) / tiles);
@@ -549,7 +555,7 @@ int Recon::pupil_vrows(int rows, std::vector<int2> *out) const {
 }
 
 size_t Recon::pupil_smem_of(int rows) const {
-    return (size_t)pupil_rows_smem_floats(rows, nxp, nps, pupil_vrows(rows), max_pos()) * sizeof(float);
+    return (size_t)pupil_rows_smem_floats(rows, nxp, nps, lhs_fused ? pupil_vrows(rows) : 0, max_pos()) * sizeof(float);
 }
 
 // Every instantiation of k_pupil_rows.
@@ -579,10 +585,11 @@ static void allow_smem(K kern, size_t smem) {
 }
 
 void Recon::set_pupil_rows(int rows) {
+    const size_t sm = pupil_smem_of(rows);
+    MB_REQUIRE(sm <= kMaxRowSmem, "pupil row block needs %zu bytes of shared memory", sm);
     std::vector<int2> v;
     pvrows = pupil_vrows(rows, &v);
-    const size_t sm = (size_t)pupil_rows_smem_floats(rows, nxp, nps, pvrows, max_pos()) * sizeof(float);
-    MB_REQUIRE(sm <= kMaxRowSmem, "pupil row block needs %zu bytes of shared memory", sm);
+    if (!lhs_fused) pvrows = 0;
     vrow.upload(v);
     prows = rows;
     ptiles = (nyp + prows - 1) / prows;
@@ -690,19 +697,19 @@ void Recon::set_hxt_rows(int rows) {
     nblk_hxt = hxt_blocks(rows);
 }
 
-PupilArgs Recon::pupil_args(bool from_x, const float *xin, int w0) const {
+PupilArgs Recon::pupil_args(bool from_x, const float *xin, int w0, bool tt_term) const {
     return PupilArgs{xin,  grad.p, tt.p,  obuf.p, hx.fwd.p, vrow.p, laytab,  wfstab,         w0,   nps, nwfs, nxp,
-                     nyp,  nxtot,  ngrad, prows,  ptiles,   pvrows, ostride, orows * ostride, from_x ? 0 : 1, act()};
+                     nyp,  nxtot,  ngrad, prows,  ptiles,   pvrows, ostride, orows * ostride, !from_x && tt_term, act()};
 }
 
 // Launch k_pupil_rows over every WFS: one launch per run of consecutive WFS
 // with the same subaperture/pupil ratio.
-void Recon::pupil_rows(bool from_x, const float *xin, cudaStream_t s) {
+void Recon::pupil_rows(bool from_x, const float *xin, cudaStream_t s, bool tt_term) {
     for (int w0 = 0; w0 < nwfs;) {
         int w1 = w0 + 1;
         while (w1 < nwfs && wfs_h[w1].pos == wfs_h[w0].pos) w1++;
         launch(pupil_kern(from_x, wfs_h[w0].pos == 2), dim3(ptiles, w1 - w0, nb), dim3(kThreads), pupil_smem, s,
-               pupil_args(from_x, xin, w0));
+               pupil_args(from_x, xin, w0, tt_term));
         w0 = w1;
     }
 }
@@ -1486,16 +1493,22 @@ void Recon::op_rhs(const float *g, float *out, cudaStream_t s) {
     hxt_rows(nullptr, out, nullptr, 0, s);
 }
 
+// The back-projected OPD of A x, what k_hxt_rows takes.
+void Recon::lhs_pupil(const float *xin, cudaStream_t s) {
+    if (lhs_fused) {  // no tip/tilt term: Hx, GP, NEA, GP^T fused per pupil-row block
+        pupil_rows(true, xin, s);
+        return;
+    }
+    // the tip/tilt projection (split 0) needs every gradient of a WFS first
+    op_hx(xin, s);
+    launch(k_gp, dim3(nblk_tt, nwfs, nb), dim3(kThreads), 0, s, opd.p, nullptr, grad.p, tt_part.p, wfs.p, nwfs, nxp, np,
+           ngrad, split ? 0 : 1, tt.p, cnt_tt.p, act());
+    pupil_rows(false, nullptr, s, !split);
+}
+
 void Recon::op_lhs(const float *xin, float *out, double *dot_part, cudaStream_t s) {
     // TomoL: Hx^T GP^T NEA^-1 (I - TT PTT) GP Hx x + L2^T L2 x   (recon_utils.c:447, tomo.cu:639)
-    if (split) {  // no tip/tilt term: Hx, GP, NEA, GP^T fused per pupil-row block
-        pupil_rows(true, xin, s);
-    } else {      // the tip/tilt projection needs every gradient of a WFS first
-        op_hx(xin, s);
-        launch(k_gp, dim3(nblk_tt, nwfs, nb), dim3(kThreads), 0, s, opd.p, nullptr, grad.p, tt_part.p, wfs.p,
-                                                          nwfs, nxp, np, ngrad, 1, tt.p, cnt_tt.p, act());
-        pupil_rows(false, nullptr, s);
-    }
+    lhs_pupil(xin, s);
     hxt_rows(xin, out, dot_part, 1, s);
 }
 
@@ -1991,7 +2004,7 @@ void Recon::time_stages(int reps, float *ms, double *bytes, int *launches) {
         // start in x, r and p is left as it was
         auto run_stage = [&]() {
             switch (st) {
-                case 0: pupil_rows(true, p.p, stream); break;
+                case 0: lhs_pupil(p.p, stream); break;
                 case 1: hxt_rows(p.p, Ap.p, pap_part.p, 1, stream); break;
                 case 2:
                     launch(k_cg_update_xr, dim3(nblk_x, nb), dim3(kThreads), 0, stream, z.p, rhs.p, p.p, Ap.p,
@@ -2332,12 +2345,12 @@ struct ReconGroup {
             launch(k_hxt_rows_group, dim3(g.start[g.n]), dim3(kHxtThreads), 0, s, g);
         }
     }
-    // A p for every member (TomoL): grouped where the tip/tilt split allows
+    // A p for every member (TomoL): grouped where its first half is one kernel
     void lhs(const std::vector<const float *> &xin, const std::vector<float *> &out, const std::vector<double *> &dot,
              cudaStream_t s) {
         std::vector<int> who;
         for (int i : order) {
-            if (m[i]->split) who.push_back(i);
+            if (m[i]->lhs_fused) who.push_back(i);
             else m[i]->op_lhs(xin[i], out[i], dot[i], s);
         }
         if (who.empty()) return;

@@ -246,6 +246,54 @@ def test_fdpcg_batch_shape_keeps_results():
         R.close()
 
 
+def test_layers_much_finer_than_the_pupil():
+    """Sixteen layers of five rows per pupil row, under a pupil 180 points
+    across: what even one pupil row touches of them does not fit a CTA's shared
+    memory, so the operator's Hx and gradients are kernels of their own (without
+    the tip/tilt term that the right-hand side has)."""
+    import dataclasses
+
+    import scipy.sparse as sps
+    from maos_b200 import config, geometry
+    from maos_b200.recon import Reconstructor
+    cfg = config.PRESETS["ltao_8m"]()
+    order = 88
+    dsa = cfg.D / order
+    cfg = dataclasses.replace(
+        cfg, atmr_dx=dsa, powfs=[dataclasses.replace(p, order=order, dsa=dsa) for p in cfg.powfs],
+        dms=[dataclasses.replace(d, dx=dsa, order=order + 1) for d in cfg.dms])
+    s = geometry.build_tomo(cfg)
+    dx = s.pmap.dx
+    assert round(s.wfs[0].dsa / dx) == 2 and 16 * 19 * s.pmap.nx * 4 > 200 * 1024 and any(w.PTT is not None for w in s.wfs)
+    ht = np.linspace(0.0, 9000.0, 16)
+    nx, ny = 24, 1000
+    xmaps = [geometry.Grid(nx, ny, 2 * dx, dx / 5, -nx * dx, -ny / 10 * dx, h) for h in ht]
+    s = dataclasses.replace(s, xmaps=xmaps, ht=ht, wt=np.full(16, 1 / 16), l2c=np.zeros(16))
+    o = TomoOracle(s)
+    o.L2 = [sps.csr_matrix((g.n, g.n)) for g in xmaps]  # l2c = 0
+    rng = np.random.default_rng(41)
+    x = rng.standard_normal((2, nx * ny * 16)) * 1e-7
+    g = rng.standard_normal((2, s.ngrad)) * 1e-6
+    R = Reconstructor(s, nbatch=2, maxit=4)
+    try:
+        got = R.apply_hx(x), R.apply_L(x), R.apply_R(g)
+        R.reset()
+        layers, _ = R.tomo(g)
+        R.autotune(reps=2)
+        again, _ = R.tomo(g)
+    finally:
+        R.close()
+    for b in range(2):
+        hx = o.hx(x[b])
+        for w in range(len(s.wfs)):
+            assert rel(got[0][b][w], hx[w]) < OP_TOL
+        assert rel(got[1][b], o.tomo_L(x[b])) < OP_TOL
+        assert rel(got[2][b], o.tomo_R(g[b])) < OP_TOL
+        want, _ = tomo_solve(o, g[b], maxit=4)
+        assert rel(layers[b], want) < SOLVE_TOL
+        assert rel(again[b], want) < SOLVE_TOL
+
+
 def test_layer_transforms_of_a_tall_layer_beside_grouped_ones():
     """Once an instance's layers outnumber the SMs, equal layers share a CTA of
     the transforms, which then tells a row pair's layer by a multiplication; a
