@@ -259,8 +259,8 @@ const float *mb_fit_solution(mb_recon *r);
  * result equals its own mb_recon_step_device's.  Members must share the
  * device and the tomography iteration count.  A member stays owned by the
  * caller and must outlive the group; after a member's tables change (updates,
- * autotune) the next step recaptures the group's graph.  At most 8 members per grouped launch (more
- * members take more launches). */
+ * autotune) the next step recaptures the group's graph.  At most 8 members per
+ * grouped launch (more members take more launches). */
 typedef struct mb_group mb_group;
 int mb_group_create(mb_recon *const *members, int n, mb_group **out);
 /* d_grad[i]: member i's FP32 gradients [nbatch_i][ngrad_i] on the device;
